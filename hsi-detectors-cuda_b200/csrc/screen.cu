@@ -9,10 +9,10 @@
 //                compacted positive list, the rest uniform over the frame;
 //   gather       features (x_b - mean_b) s_b rounded to bfloat16, band-major
 //                [Bp][n], and the 0/1 labels from the score map;
-//   forward      one thread per sample (bfloat16 weights, FP32 accumulation,
-//                h1 rounded to bfloat16 as inference does), storing the
-//                activations and back-propagated deltas;
-//   gradients    dW = delta^T act as small deterministic SIMT GEMMs;
+//   gradients    forward (bfloat16 weights, FP32 accumulation, h1 rounded to
+//                bfloat16 as inference does), deltas and dW = delta^T act in
+//                one kernel over chunks of samples; per-CTA partials added in
+//                a fixed order;
 //   adam         FP32 master weights; the forward reads them rounded.
 // Inference (screen_tc_kernel, below) runs layers 1 and 2 on the tensor
 // cores straight from the fp16 cube.
@@ -21,6 +21,8 @@
 //   W1[64][Bp] | b1[64] | W2[32][64] | b2[32] | w3[32] | b3
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
+
+#include <type_traits>
 
 #include "synth.h"
 #include "launch_state.h"
@@ -135,173 +137,373 @@ __global__ void gather_kernel(const T* __restrict__ cube, int64_t stride, int B,
   features[static_cast<int64_t>(b) * n + s] = v;
 }
 
-// ---- forward + deltas, one thread per sample --------------------------------
-// Activations and deltas, sample-minor: H1[64][n], H2[32][n], D1[64][n],
-// D2[32][n], D3[n]; per-block partial losses.
-struct Acts {
-  float *H1, *H2, *D1, *D2, *D3, *loss_part;
+// ---- one training pass: forward, deltas and gradient partials ----------------
+//
+// A CTA takes chunks of S samples with the whole network in shared memory:
+// the chunk's features, W1 and W2 rounded to bfloat16, and the activations
+// and deltas, which never reach global memory.  All five products run from
+// shared memory in FP32 register tiles; the weight gradients stay in registers
+// over a CTA's chunks, and each CTA writes one partial of every parameter that
+// reduce_kernel adds in a fixed order (deterministic, and shorter sums than
+// one chain over the batch).
+// 8192 samples of 224 bands: 28 us here and 3.4 us in reduce_kernel, where a
+// one-thread-per-sample forward, six row-dot launches (20 blocks, each one
+// chain over the whole batch) and a loss launch took 1.58 ms.
+// Bound: shared-memory reads, then FP32 FMA.  Layer 1 and dW1 are 64 x Bp products per sample each,
+// 7.5 us on 128 SMs for 8192 samples of 224 bands; the tiles read one shared
+// value per 8 (layer 1) or 16 (dW1) FMAs, so shared memory keeps up.  S = 64
+// amortises the 64 KB of W1 a CTA stages; 32 up to 4736 samples (148 chunks),
+// where 64 would leave more than half of the SMs without one.
+constexpr int kTrainThreads = 256;
+constexpr int kTrainMaxCtas = 148;  // partials in the workspace; more chunks than that are looped over
+constexpr int kW1Stride = kH1 + 2;  // W1^T rows [b][64]: 2-way conflicts on the transposing store, float2 reads
+constexpr int kW2Stride = kH2 + 4;  // W2^T rows [j][32]: float4 reads along k
+
+__host__ __device__ inline int train_chunk(int n) { return n <= 32 * kTrainMaxCtas ? 32 : 64; }
+__host__ __device__ inline int train_ctas(int n) {
+  const int chunks = (n + train_chunk(n) - 1) / train_chunk(n);
+  return chunks < kTrainMaxCtas ? chunks : kTrainMaxCtas;
+}
+// floats of one CTA's partial: every parameter, then the loss sum, padded to 128 bytes
+__host__ __device__ inline int64_t partial_stride(int B) { return (param_count(B) + 1 + 31) / 32 * 32; }
+
+template <int S>
+struct TrainSmem {
+  static constexpr int kS = S + 4;  // sample-minor rows: 16-byte aligned, 8 rows apart in the banks
+  static __host__ __device__ constexpr int floats(int bp) {
+    return bp * kS + bp * kW1Stride + kH1 * kW2Stride + kH1 * kS /* h1 */ + S * (kH1 + 4) /* delta1^T */ +
+           2 * kH2 * kS /* z2 -> delta2, h2 */ + 2 * S /* delta3, loss */ + kH1 + 2 * kH2 /* b1, b2, w3 */;
+  }
 };
 
-constexpr int kFwdThreads = 128;
+__device__ __forceinline__ void cp_async16(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 16 : 0)
+               : "memory");
+}
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool valid) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_addr(dst)), "l"(src), "r"(valid ? 4 : 0)
+               : "memory");
+}
 
-__global__ void __launch_bounds__(kFwdThreads) forward_kernel(const float* __restrict__ params, int B,
-                                                             const float* __restrict__ X,
-                                                             const float* __restrict__ labels, int n,
-                                                             float pos_weight, Acts a) {
-  extern __shared__ float sw[];
-  const int Bp = padded_bands(B);
+// NB = Bp / 64.  `vec`: the features' rows start on 16 bytes (n a multiple of 4).
+template <int NB, int S>
+__global__ void __launch_bounds__(kTrainThreads, 1)
+    train_kernel(const float* __restrict__ params, int B, const float* __restrict__ X,
+                 const float* __restrict__ labels, int n, float pos_weight, int vec, float* __restrict__ partials) {
+  constexpr int Bp = 64 * NB;
+  constexpr int kS = TrainSmem<S>::kS;
+  constexpr int kD = kH1 + 4;  // delta1^T row: [s][64]
+  extern __shared__ __align__(16) float sw[];
+  float* xs = sw;                         // [Bp][kS]
+  float* w1t = xs + Bp * kS;              // [Bp][kW1Stride], bfloat16 values
+  float* w2t = w1t + Bp * kW1Stride;      // [64][kW2Stride], bfloat16 values
+  float* h1 = w2t + kH1 * kW2Stride;      // [64][kS]
+  float* d1t = h1 + kH1 * kS;             // [S][kD]
+  float* d2 = d1t + S * kD;               // [32][kS]: z2, then delta2
+  float* h2 = d2 + kH2 * kS;              // [32][kS]
+  float* d3 = h2 + kH2 * kS;              // [S]
+  float* ls = d3 + S;                     // [S]
+  float* b1 = ls + S;
+  float* b2 = b1 + kH1;
+  float* w3 = b2 + kH2;
   const ParamView v = view(const_cast<float*>(params), B);
-  // W1 transposed to [b][64] and W2 to [j][32], both rounded to bfloat16
-  float* w1t = sw;
-  float* w2t = w1t + static_cast<int64_t>(Bp) * kH1;
-  float* w3r = w2t + kH1 * kH2;
-  __shared__ float s_loss[kFwdThreads / 32];
-  for (int e = threadIdx.x; e < Bp * kH1; e += blockDim.x) {
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int chunks = (n + S - 1) / S;
+
+  auto load_features = [&](int chunk) {
+    const int s0 = chunk * S;
+    if (vec) {
+      for (int e = tid; e < Bp * (S / 4); e += kTrainThreads) {
+        const int b = e / (S / 4), s = e % (S / 4) * 4;
+        const bool in = s0 + s < n;
+        cp_async16(xs + b * kS + s, X + static_cast<int64_t>(b) * n + (in ? s0 + s : 0), in);
+      }
+    } else {
+      for (int e = tid; e < Bp * S; e += kTrainThreads) {
+        const int b = e / S, s = e % S;
+        const bool in = s0 + s < n;
+        cp_async4(xs + b * kS + s, X + static_cast<int64_t>(b) * n + (in ? s0 + s : 0), in);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_features(blockIdx.x);
+#pragma unroll 16
+  for (int e = tid; e < Bp * kH1; e += kTrainThreads) {  // 16 loads in flight a thread
     const int j = e / Bp, b = e % Bp;
-    w1t[b * kH1 + j] = bf16r(v.W1[e]);
+    w1t[b * kW1Stride + j] = bf16r(v.W1[e]);
   }
-  for (int e = threadIdx.x; e < kH2 * kH1; e += blockDim.x) {
-    const int k = e / kH1, j = e % kH1;
-    w2t[j * kH2 + k] = bf16r(v.W2[e]);
+  for (int e = tid; e < kH2 * kH1; e += kTrainThreads) w2t[(e % kH1) * kW2Stride + e / kH1] = bf16r(v.W2[e]);
+  if (tid < kH1) b1[tid] = v.b1[tid];
+  if (tid < kH2) {
+    b2[tid] = v.b2[tid];
+    w3[tid] = bf16r(v.w3[tid]);
   }
-  for (int k = threadIdx.x; k < kH2; k += blockDim.x) w3r[k] = bf16r(v.w3[k]);
-  __syncthreads();
-  const int s = blockIdx.x * blockDim.x + threadIdx.x;
-  float loss = 0.0f;
-  if (s < n) {
-    float z1[kH1];
-#pragma unroll
-    for (int j = 0; j < kH1; ++j) z1[j] = v.b1[j];
-    for (int b = 0; b < B; ++b) {
-      const float x = X[static_cast<int64_t>(b) * n + s];
-      const float4* w = reinterpret_cast<const float4*>(w1t + b * kH1);
-#pragma unroll
-      for (int q = 0; q < kH1 / 4; ++q) {
-        const float4 c = w[q];
-        z1[4 * q] = fmaf(c.x, x, z1[4 * q]);
-        z1[4 * q + 1] = fmaf(c.y, x, z1[4 * q + 1]);
-        z1[4 * q + 2] = fmaf(c.z, x, z1[4 * q + 2]);
-        z1[4 * q + 3] = fmaf(c.w, x, z1[4 * q + 3]);
-      }
-    }
-#pragma unroll
-    for (int j = 0; j < kH1; ++j) a.H1[static_cast<int64_t>(j) * n + s] = bf16r(fmaxf(z1[j], 0.0f));
-    // layer 2 re-reads h1 (this thread's own writes) instead of keeping z1 live
-    float z2[kH2];
-#pragma unroll
-    for (int k = 0; k < kH2; ++k) z2[k] = v.b2[k];
-#pragma unroll 1
-    for (int j = 0; j < kH1; ++j) {
-      const float h = a.H1[static_cast<int64_t>(j) * n + s];
-      const float4* w = reinterpret_cast<const float4*>(w2t + j * kH2);
-#pragma unroll
-      for (int q = 0; q < kH2 / 4; ++q) {
-        const float4 c = w[q];
-        z2[4 * q] = fmaf(c.x, h, z2[4 * q]);
-        z2[4 * q + 1] = fmaf(c.y, h, z2[4 * q + 1]);
-        z2[4 * q + 2] = fmaf(c.z, h, z2[4 * q + 2]);
-        z2[4 * q + 3] = fmaf(c.w, h, z2[4 * q + 3]);
-      }
-    }
-    float z3 = v.b3[0];
-#pragma unroll
-    for (int k = 0; k < kH2; ++k) {
-      const float h2 = fmaxf(z2[k], 0.0f);
-      a.H2[static_cast<int64_t>(k) * n + s] = h2;
-      z3 = fmaf(w3r[k], h2, z3);
-    }
-    const float y = labels[s], w = y > 0.5f ? pos_weight : 1.0f;
-    const float sp = z3 > 0.0f ? z3 + log1pf(expf(-z3)) : log1pf(expf(z3));
-    loss = w * (sp - y * z3);
-    const float d3 = w * (1.0f / (1.0f + expf(-z3)) - y) / static_cast<float>(n);
-    a.D3[s] = d3;
-    float d2[kH2];
-#pragma unroll
-    for (int k = 0; k < kH2; ++k) {
-      d2[k] = z2[k] > 0.0f ? d3 * w3r[k] : 0.0f;
-      a.D2[static_cast<int64_t>(k) * n + s] = d2[k];
-    }
-    // delta1_j = [z1_j > 0] sum_k delta2_k W2_kj  (h1_j > 0 exactly when z1_j > 0)
-#pragma unroll 1
-    for (int j = 0; j < kH1; ++j) {
-      const float4* w2 = reinterpret_cast<const float4*>(w2t + j * kH2);
-      float acc = 0.0f;
-#pragma unroll
-      for (int q = 0; q < kH2 / 4; ++q) {
-        const float4 c = w2[q];
-        acc = fmaf(d2[4 * q], c.x, acc);
-        acc = fmaf(d2[4 * q + 1], c.y, acc);
-        acc = fmaf(d2[4 * q + 2], c.z, acc);
-        acc = fmaf(d2[4 * q + 3], c.w, acc);
-      }
-      const float h = a.H1[static_cast<int64_t>(j) * n + s];
-      a.D1[static_cast<int64_t>(j) * n + s] = h > 0.0f ? acc : 0.0f;
-    }
-  }
-  // block partial of the loss (fixed order: deterministic)
-  for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xffffffffu, loss, o);
-  if ((threadIdx.x & 31) == 0) s_loss[threadIdx.x >> 5] = loss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    float t = 0.0f;
-    for (int w = 0; w < kFwdThreads / 32; ++w) t += s_loss[w];
-    a.loss_part[blockIdx.x] = t;
-  }
-}
+  const float b3 = v.b3[0];
 
-// C[M][N] = A[M][K] B[N][K]^T (both K-contiguous, K = samples); 32 x 32 output
-// tiles, 256 threads, 4 outputs each; fixed summation order.
-__global__ void __launch_bounds__(256) rowdot_kernel(const float* __restrict__ A, const float* __restrict__ Bm, int M,
-                                                     int N, int K, float* __restrict__ C, int ldc) {
-  __shared__ float sa[32][33];
-  __shared__ float sb[32][33];
-  const int m0 = blockIdx.y * 32, n0 = blockIdx.x * 32;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // ty 0..7: rows ty, ty+8, ty+16, ty+24
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-  for (int k0 = 0; k0 < K; k0 += 32) {
-    for (int r = ty; r < 32; r += 8) {
-      const int k = k0 + tx;
-      sa[r][tx] = (m0 + r < M && k < K) ? A[static_cast<int64_t>(m0 + r) * K + k] : 0.0f;
-      sb[r][tx] = (n0 + r < N && k < K) ? Bm[static_cast<int64_t>(n0 + r) * K + k] : 0.0f;
+  // gradients of this CTA: dW1 rows 8 warp .. + 7 by columns lane + 32 i (row
+  // pairs packed), dW2 rows 4 warp .. + 3 by columns lane and lane + 32, and
+  // one bias / w3 / loss element on each of the first threads
+  float2 g1[4][2 * NB];
+  float g2[4][2];
+  float gs = 0.0f;
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+#pragma unroll
+    for (int i = 0; i < 2 * NB; ++i) g1[r][i] = make_float2(0.0f, 0.0f);
+    g2[r][0] = g2[r][1] = 0.0f;
+  }
+
+  for (int chunk = blockIdx.x; chunk < chunks; chunk += gridDim.x) {
+    const int s0 = chunk * S;
+    if (chunk != static_cast<int>(blockIdx.x)) {
+      __syncthreads();  // the previous chunk's features and deltas are done with
+      load_features(chunk);
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
+
+    // layer 1: 4 hidden units x S/16 samples a thread, bands in order
+    {
+      constexpr int kQ = S / 16;
+      const int ss = (tid & 15) * kQ, j0 = (tid >> 4) * 4;
+      float2 z[2][kQ];
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        z[0][q] = make_float2(b1[j0], b1[j0 + 1]);
+        z[1][q] = make_float2(b1[j0 + 2], b1[j0 + 3]);
+      }
 #pragma unroll 8
-    for (int k = 0; k < 32; ++k) {
-      const float bv = sb[tx][k];
+      for (int b = 0; b < B; ++b) {
+        const float2 wa = *reinterpret_cast<const float2*>(w1t + b * kW1Stride + j0);
+        const float2 wb = *reinterpret_cast<const float2*>(w1t + b * kW1Stride + j0 + 2);
+        float x[kQ];
+        if constexpr (kQ == 4) {
+          const float4 t = *reinterpret_cast<const float4*>(xs + b * kS + ss);
+          x[0] = t.x, x[1] = t.y, x[2] = t.z, x[3] = t.w;
+        } else {
+          const float2 t = *reinterpret_cast<const float2*>(xs + b * kS + ss);
+          x[0] = t.x, x[1] = t.y;
+        }
 #pragma unroll
-      for (int i = 0; i < 4; ++i) acc[i] = fmaf(sa[ty + 8 * i][k], bv, acc[i]);
+        for (int q = 0; q < kQ; ++q) {
+          const float2 xx = make_float2(x[q], x[q]);
+          z[0][q] = ffma2(wa, xx, z[0][q]);
+          z[1][q] = ffma2(wb, xx, z[1][q]);
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < kQ; ++q) {
+        const bool in = s0 + ss + q < n;
+        h1[j0 * kS + ss + q] = in ? bf16r(fmaxf(z[0][q].x, 0.0f)) : 0.0f;
+        h1[(j0 + 1) * kS + ss + q] = in ? bf16r(fmaxf(z[0][q].y, 0.0f)) : 0.0f;
+        h1[(j0 + 2) * kS + ss + q] = in ? bf16r(fmaxf(z[1][q].x, 0.0f)) : 0.0f;
+        h1[(j0 + 3) * kS + ss + q] = in ? bf16r(fmaxf(z[1][q].y, 0.0f)) : 0.0f;
+      }
     }
     __syncthreads();
-  }
+    // layer 2: 4 units x S/32 samples a thread
+    {
+      constexpr int kQ = S / 32;
+      const int k0 = warp * 4;
+      float z[4][kQ];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int m = m0 + ty + 8 * i, nn = n0 + tx;
-    if (m < M && nn < N) C[static_cast<int64_t>(m) * ldc + nn] = acc[i];
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) z[k][q] = b2[k0 + k];
+#pragma unroll 8
+      for (int j = 0; j < kH1; ++j) {
+        const float4 w = *reinterpret_cast<const float4*>(w2t + j * kW2Stride + k0);
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          const float h = h1[j * kS + lane + 32 * q];
+          z[0][q] = fmaf(w.x, h, z[0][q]);
+          z[1][q] = fmaf(w.y, h, z[1][q]);
+          z[2][q] = fmaf(w.z, h, z[2][q]);
+          z[3][q] = fmaf(w.w, h, z[3][q]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          d2[(k0 + k) * kS + lane + 32 * q] = z[k][q];
+          h2[(k0 + k) * kS + lane + 32 * q] = fmaxf(z[k][q], 0.0f);
+        }
+    }
+    __syncthreads();
+    // layer 3, the loss and delta3: one thread a sample
+    if (tid < S) {
+      const bool in = s0 + tid < n;
+      float z3 = b3;
+#pragma unroll
+      for (int k = 0; k < kH2; ++k) z3 = fmaf(w3[k], h2[k * kS + tid], z3);
+      const float y = in ? labels[s0 + tid] : 0.0f, w = y > 0.5f ? pos_weight : 1.0f;
+      const float sp = z3 > 0.0f ? z3 + log1pf(expf(-z3)) : log1pf(expf(z3));
+      ls[tid] = in ? w * (sp - y * z3) : 0.0f;
+      d3[tid] = in ? w * (1.0f / (1.0f + expf(-z3)) - y) / static_cast<float>(n) : 0.0f;
+    }
+    __syncthreads();
+    for (int e = tid; e < kH2 * S; e += kTrainThreads) {
+      const int k = e / S, s = e % S;
+      const float z = d2[k * kS + s];
+      d2[k * kS + s] = (z > 0.0f && s0 + s < n) ? d3[s] * w3[k] : 0.0f;
+    }
+    __syncthreads();
+    // delta1_j = [h1_j > 0] sum_k delta2_k W2_kj: 8 units (4 rows of two warps' halves) x S/32 samples a thread
+    {
+      constexpr int kQ = S / 32;
+      const int j0 = warp * 8;
+#pragma unroll
+      for (int jj = 0; jj < 8; jj += 4) {
+        float acc[4][kQ];
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int q = 0; q < kQ; ++q) acc[j][q] = 0.0f;
+#pragma unroll 2
+        for (int k = 0; k < kH2; k += 4) {
+          float w[4][4];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float4 t = *reinterpret_cast<const float4*>(w2t + (j0 + jj + j) * kW2Stride + k);
+            w[j][0] = t.x, w[j][1] = t.y, w[j][2] = t.z, w[j][3] = t.w;
+          }
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+            for (int q = 0; q < kQ; ++q) {
+              const float d = d2[(k + kk) * kS + lane + 32 * q];
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[j][q] = fmaf(d, w[j][kk], acc[j][q]);
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kQ; ++q) {
+          const int s = lane + 32 * q;
+          float4 t;
+          t.x = h1[(j0 + jj) * kS + s] > 0.0f ? acc[0][q] : 0.0f;
+          t.y = h1[(j0 + jj + 1) * kS + s] > 0.0f ? acc[1][q] : 0.0f;
+          t.z = h1[(j0 + jj + 2) * kS + s] > 0.0f ? acc[2][q] : 0.0f;
+          t.w = h1[(j0 + jj + 3) * kS + s] > 0.0f ? acc[3][q] : 0.0f;
+          *reinterpret_cast<float4*>(d1t + s * kD + j0 + jj) = t;
+        }
+      }
+    }
+    __syncthreads();
+    // dW1 += delta1 X^T, four samples at a time: X by float4 along the samples
+    // (rows of kS floats: 8 lanes cover the banks), delta1 broadcast
+#pragma unroll 1
+    for (int s = 0; s < S; s += 4) {
+      float2 d[4][4];  // [sample][row pair]
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float4 a = *reinterpret_cast<const float4*>(d1t + (s + q) * kD + warp * 8);
+        const float4 c = *reinterpret_cast<const float4*>(d1t + (s + q) * kD + warp * 8 + 4);
+        d[q][0] = make_float2(a.x, a.y), d[q][1] = make_float2(a.z, a.w);
+        d[q][2] = make_float2(c.x, c.y), d[q][3] = make_float2(c.z, c.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 2 * NB; ++i) {
+        const float4 x = *reinterpret_cast<const float4*>(xs + (lane + 32 * i) * kS + s);
+        const float xq[4] = {x.x, x.y, x.z, x.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+          const float2 xx = make_float2(xq[q], xq[q]);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) g1[r][i] = ffma2(d[q][r], xx, g1[r][i]);
+        }
+      }
+    }
+    // dW2 += delta2 h1^T, the same way
+#pragma unroll 2
+    for (int s = 0; s < S; s += 4) {
+      const float4 ha = *reinterpret_cast<const float4*>(h1 + lane * kS + s);
+      const float4 hb = *reinterpret_cast<const float4*>(h1 + (lane + 32) * kS + s);
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float4 d = *reinterpret_cast<const float4*>(d2 + (warp * 4 + r) * kS + s);
+        g2[r][0] = fmaf(d.w, ha.w, fmaf(d.z, ha.z, fmaf(d.y, ha.y, fmaf(d.x, ha.x, g2[r][0]))));
+        g2[r][1] = fmaf(d.w, hb.w, fmaf(d.z, hb.z, fmaf(d.y, hb.y, fmaf(d.x, hb.x, g2[r][1]))));
+      }
+    }
+    // db1 (threads 0..63), db2 (64..95), dw3 (96..127), db3 (128), loss (160)
+    if (tid < kH1) {
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) gs += d1t[s * kD + tid];
+    } else if (tid < kH1 + kH2) {
+      const float* r = d2 + (tid - kH1) * kS;
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) gs += r[s];
+    } else if (tid < kH1 + 2 * kH2) {
+      const float* r = h2 + (tid - kH1 - kH2) * kS;
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) gs = fmaf(d3[s], s0 + s < n ? r[s] : 0.0f, gs);
+    } else if (tid == kH1 + 2 * kH2 || tid == kH1 + 3 * kH2) {
+      const float* r = tid == kH1 + 2 * kH2 ? d3 : ls;
+#pragma unroll 8
+      for (int s = 0; s < S; ++s) gs += r[s];
+    }
   }
+
+  const ParamView g = view(partials + static_cast<int64_t>(blockIdx.x) * partial_stride(B), B);
+#pragma unroll
+  for (int i = 0; i < 2 * NB; ++i)
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      g.W1[(warp * 8 + 2 * r) * Bp + lane + 32 * i] = g1[r][i].x;
+      g.W1[(warp * 8 + 2 * r + 1) * Bp + lane + 32 * i] = g1[r][i].y;
+    }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    g.W2[(warp * 4 + r) * kH1 + lane] = g2[r][0];
+    g.W2[(warp * 4 + r) * kH1 + lane + 32] = g2[r][1];
+  }
+  if (tid < kH1) g.b1[tid] = gs;
+  else if (tid < kH1 + kH2) g.b2[tid - kH1] = gs;
+  else if (tid < kH1 + 2 * kH2) g.w3[tid - kH1 - kH2] = gs;
+  else if (tid == kH1 + 2 * kH2) g.b3[0] = gs;
+  else if (tid == kH1 + 3 * kH2) g.b3[1] = gs;
 }
 
-// out[r] = sum_k A[r][k], one block per row.
-__global__ void __launch_bounds__(256) rowsum_kernel(const float* __restrict__ A, int K, float* __restrict__ out) {
-  __shared__ float s[8];
-  const float* a = A + static_cast<int64_t>(blockIdx.x) * K;
+// out[i] = sum over the CTAs' partials; 32 parameters by 8 slices of the
+// partials a block, so a thread has its few loads in flight together (one
+// thread per parameter would chain 128 of them).  The element after the last
+// parameter is the loss sum.
+__global__ void __launch_bounds__(256) reduce_kernel(const float* __restrict__ partials, int nparts, int64_t stride,
+                                                    int64_t count, int n, float* __restrict__ grads,
+                                                    float* __restrict__ loss) {
+  __shared__ float s[8][33];
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * 32 + lane;
   float t = 0.0f;
-  for (int k = threadIdx.x; k < K; k += blockDim.x) t += a[k];
-  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = t;
+  if (i <= count) {
+#pragma unroll 8
+    for (int c = slice; c < nparts; c += 8) t += partials[c * stride + i];
+  }
+  s[slice][lane] = t;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float r = 0.0f;
-    for (int w = 0; w < 8; ++w) r += s[w];
-    out[blockIdx.x] = r;
+  if (slice == 0 && i <= count) {
+    float r = s[0][lane];
+#pragma unroll
+    for (int w = 1; w < 8; ++w) r += s[w][lane];
+    if (i < count) grads[i] = r;
+    else if (loss) *loss = r / static_cast<float>(n);
   }
 }
 
-__global__ void loss_kernel(const float* __restrict__ part, int nparts, int n, float* __restrict__ loss) {
-  if (threadIdx.x == 0 && blockIdx.x == 0) {
-    float t = 0.0f;
-    for (int i = 0; i < nparts; ++i) t += part[i];
-    *loss = t / static_cast<float>(n);
-  }
+template <int NB, int S>
+cudaError_t launch_train(const float* params, int B, const float* X, const float* labels, int n, float pos_weight,
+                         int vec, float* partials, cudaStream_t s) {
+  constexpr int smem = static_cast<int>(sizeof(float)) * TrainSmem<S>::floats(64 * NB);
+  const cudaError_t e = raise_smem_limit(train_kernel<NB, S>, smem);
+  if (e != cudaSuccess) return e;
+  train_kernel<NB, S><<<train_ctas(n), kTrainThreads, smem, s>>>(params, B, X, labels, n, pos_weight, vec, partials);
+  return cudaGetLastError();
+}
+
+size_t train_bytes(int B, int n) {
+  return sizeof(float) * static_cast<size_t>(train_ctas(n)) * static_cast<size_t>(partial_stride(B)) + 256;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
@@ -316,26 +518,6 @@ __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float*
     v[i] = vi;
     p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
   }
-}
-
-struct TrainWs {
-  Acts acts;
-  size_t bytes;
-};
-
-TrainWs carve_train(void* ws, int n) {
-  TrainWs t;
-  float* f = static_cast<float*>(ws);
-  const int64_t nn = n;
-  t.acts.H1 = f;
-  t.acts.H2 = t.acts.H1 + kH1 * nn;
-  t.acts.D1 = t.acts.H2 + kH2 * nn;
-  t.acts.D2 = t.acts.D1 + kH1 * nn;
-  t.acts.D3 = t.acts.D2 + kH2 * nn;
-  t.acts.loss_part = t.acts.D3 + nn;
-  const int64_t parts = (nn + kFwdThreads - 1) / kFwdThreads;
-  t.bytes = sizeof(float) * static_cast<size_t>((2 * kH1 + 2 * kH2 + 1) * nn + parts) + 256;
-  return t;
 }
 
 // ---- inference on the tensor cores -------------------------------------------
@@ -711,7 +893,7 @@ extern "C" HSI_API int hsi_screen_gather(const void* d_cube, int dtype, int64_t 
 
 extern "C" HSI_API size_t hsi_screen_train_workspace_bytes(int bands, int n) {
   if (bands <= 0 || n <= 0) return 0;
-  return carve_train(nullptr, n).bytes;
+  return train_bytes(bands, n);
 }
 
 extern "C" HSI_API int hsi_screen_gradients(const float* d_params, int bands, const float* d_features,
@@ -720,26 +902,28 @@ extern "C" HSI_API int hsi_screen_gradients(const float* d_params, int bands, co
                                             hsi_stream_t stream) {
   if (!d_params || !d_features || !d_labels || !d_grads || n <= 0 || bands <= 0 || bands > HSI_MAX_BANDS)
     return HSI_E_INVALID;
-  const TrainWs t = carve_train(d_workspace, n);
-  if (!d_workspace || workspace_bytes < t.bytes) return HSI_E_WORKSPACE;
+  if (!d_workspace || workspace_bytes < train_bytes(bands, n)) return HSI_E_WORKSPACE;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const int Bp = padded_bands(bands);
-  const size_t smem = sizeof(float) * (static_cast<size_t>(Bp) * kH1 + kH1 * kH2 + kH2);
-  // the largest band count's layout, set once per device
-  const cudaError_t configured =
-      raise_smem_limit(forward_kernel, static_cast<int>(sizeof(float) * (256 * kH1 + kH1 * kH2 + kH2)));
-  if (configured != cudaSuccess) return static_cast<int>(configured);
-  const int blocks = (n + kFwdThreads - 1) / kFwdThreads;
-  forward_kernel<<<blocks, kFwdThreads, smem, s>>>(d_params, bands, d_features, d_labels, n, pos_weight, t.acts);
-  const ParamView g = view(d_grads, bands);
-  // dW1 = D1 X^T [64][Bp], dW2 = D2 H1^T [32][64], dw3 = D3 H2^T [1][32]
-  rowdot_kernel<<<dim3((Bp + 31) / 32, 2), 256, 0, s>>>(t.acts.D1, d_features, kH1, Bp, n, g.W1, Bp);
-  rowdot_kernel<<<dim3(2, 1), 256, 0, s>>>(t.acts.D2, t.acts.H1, kH2, kH1, n, g.W2, kH1);
-  rowdot_kernel<<<dim3(1, 1), 256, 0, s>>>(t.acts.D3, t.acts.H2, 1, kH2, n, g.w3, kH2);
-  rowsum_kernel<<<kH1, 256, 0, s>>>(t.acts.D1, n, g.b1);
-  rowsum_kernel<<<kH2, 256, 0, s>>>(t.acts.D2, n, g.b2);
-  rowsum_kernel<<<1, 256, 0, s>>>(t.acts.D3, n, g.b3);
-  if (d_loss) loss_kernel<<<1, 32, 0, s>>>(t.acts.loss_part, blocks, n, d_loss);
+  float* partials = static_cast<float*>(d_workspace);
+  // 16-byte feature copies need every row on 16 bytes
+  const int vec = (n & 3) == 0 && (reinterpret_cast<uintptr_t>(d_features) & 15u) == 0;
+  const auto launch = [&](auto nb) {
+    constexpr int NB = decltype(nb)::value;
+    return train_chunk(n) == 32
+               ? launch_train<NB, 32>(d_params, bands, d_features, d_labels, n, pos_weight, vec, partials, s)
+               : launch_train<NB, 64>(d_params, bands, d_features, d_labels, n, pos_weight, vec, partials, s);
+  };
+  cudaError_t e;
+  switch (padded_bands(bands) / 64) {
+    case 1: e = launch(std::integral_constant<int, 1>{}); break;
+    case 2: e = launch(std::integral_constant<int, 2>{}); break;
+    case 3: e = launch(std::integral_constant<int, 3>{}); break;
+    default: e = launch(std::integral_constant<int, 4>{}); break;
+  }
+  if (e != cudaSuccess) return static_cast<int>(e);
+  const int64_t count = param_count(bands);
+  reduce_kernel<<<static_cast<int>(count / 32 + 1), 256, 0, s>>>(partials, train_ctas(n), partial_stride(bands), count,
+                                                                 n, d_grads, d_loss);
   return static_cast<int>(cudaGetLastError());
 }
 

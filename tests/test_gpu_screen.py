@@ -72,6 +72,46 @@ def test_gradients_match_oracle(hsi, orc, B, n):
         off += size
 
 
+@pytest.mark.parametrize("B,n,off", [(224, 1, 0), (16, 31, 0), (64, 33, 1), (65, 4736, 0), (129, 4740, 0),
+                                     (256, 4739, 0), (224, 9541, 0), (200, 9600, 1)])
+def test_gradients_over_sample_chunks(hsi, orc, B, n, off):
+    """One sample, chunks with a tail, both chunk sizes (32 samples up to 4736,
+    64 above), more chunks than CTAs (from 9473), every padded band count, and
+    features whose rows do not start on 16 bytes (n not a multiple of 4, or a
+    base `off` floats into an allocation).  Tolerance as above: the h1 of one
+    unit may round to the other bfloat16 neighbour (2^-8 of it)."""
+    L = hsi.lib()
+    p, Bp = _params(hsi, B, 31 + B)
+    rng = np.random.default_rng(B + n)
+    feats = np.zeros((Bp, n), np.float32)
+    feats[:B] = _bf16(rng.standard_normal((B, n)) * 1.5)
+    labels = (rng.random(n) < 0.2).astype(np.float32)
+    store = torch.zeros(Bp * n + off, device="cuda")
+    store[off:] = torch.from_numpy(feats).cuda().reshape(-1)
+    X, y = store[off:], torch.from_numpy(labels).cuda()
+    wb = L.hsi_screen_train_workspace_bytes(B, n)
+    ws = torch.empty(wb, dtype=torch.uint8, device="cuda")
+    grads = [torch.full_like(p, np.nan) for _ in range(2)]
+    loss = torch.zeros(1, device="cuda")
+    for g in grads:
+        assert L.hsi_screen_gradients(_p(p), B, _p(X), _p(y), n, C.c_float(3.0), _p(g), _p(loss), _p(ws), wb,
+                                      None) == 0
+    assert L.hsi_screen_gradients(_p(p), B, _p(X), _p(y), n, C.c_float(3.0), _p(g), None, _p(ws), wb - 1,
+                                  None) == hsi.E_WORKSPACE
+    torch.cuda.synchronize()
+    assert torch.equal(grads[0], grads[1])  # fixed summation order
+    _, loss0, g0 = orc.mlp(p.cpu().numpy(), B, feats[:B].T.copy(), labels, pos_weight=3.0, round_bf16=True,
+                           grads=True)
+    g = grads[0].cpu().numpy().astype(np.float64)
+    assert abs(float(loss.item()) - loss0) <= 1e-5 * abs(loss0)
+    pos = 0
+    for name, size in (("W1", 64 * Bp), ("b1", 64), ("W2", 2048), ("b2", 32), ("w3", 32), ("b3", 1)):
+        a, b = g[pos:pos + size], g0[pos:pos + size]
+        err = np.linalg.norm(a - b) / max(np.linalg.norm(b), 1e-30)
+        assert err <= 2e-3, f"{name}: {err:.3e}"
+        pos += size
+
+
 def test_adam_step_moves_against_the_gradient(hsi):
     L = hsi.lib()
     B = 16

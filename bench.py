@@ -454,7 +454,7 @@ class Workload:
             events[1].record(stream)
         self.counts.zero_()
         hsi.detect_batch(self.jobs, self.det_ws, stream=stream)
-        launches += 3
+        launches += 2
         if events is not None and len(events) > 3:
             events[3].record(stream)
         return launches
@@ -1228,7 +1228,7 @@ def measure_screen(args, dist, world, rank, device):
                                vp(dets), vp(dcount), vp(dws), dws.numel(), s), "final list")
         if ev:
             ev[2].record(stream)
-        return 11 + 6
+        return 9 + 6
 
     def plain_step(src, ev=None):
         if ev:
@@ -1433,8 +1433,8 @@ def run_batch(args):
     ms, eager_ms = max_over_ranks(dist, [ms, eager_ms], device)
     tuning = batch.tuning()
     # launches per run: demosaic, moments (6 tensor-core / 3 plain), factor, RX/ACE (prep + main per pass),
-    # one scorer launch, the counts memset, three detection launches per 64 lists
-    launches = 1 + 3 * ((3 * BATCH_FRAMES + 63) // 64)
+    # one scorer launch, the counts memset, two detection launches per 64 lists
+    launches = 1 + 2 * ((3 * BATCH_FRAMES + 63) // 64)
     for (h, w, b, t, mosaic) in specs:
         launches += (1 if mosaic else 0) + (6 if (b <= 127 and h * w >= 32768) else 3) + 1
         launches += 2 * (1 if b > 127 else -(-t // max(1, min(16, 128 - b))))

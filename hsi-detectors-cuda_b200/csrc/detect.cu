@@ -1,34 +1,31 @@
 // detect.cu - threshold + non-maximum suppression + ordered compaction.
 //
-// Three launches for a whole batch of score maps, no atomics on the data
-// path, so every list comes out in raster order and is identical run to run:
-//   1. flags:  per tile of 256 columns x 64 rows of one map, every pixel's
-//              pass/fail as warp ballot words (a bitmask in the workspace:
-//              one word per 32 pixels of a 2048-pixel row segment).  The
-//              map's rows stream through a shared-memory ring (cp.async, four
-//              rows ahead).  Per row, each column's first-best score of the
-//              (2r+1)-row window (better score, then lower row) is found
-//              once; a candidate passes when none of the 2r+1 column bests
-//              around it comes first in the window's order (better score,
-//              then lower linear index).  Out-of-frame neighbours are NaN,
-//              which never win or tie, exactly like the bounds checks of the
-//              CPU loop.  Radii above 8 read each candidate's window from
-//              global memory instead.  Maps of radius <= 4 whose width is a
-//              multiple of 4 (and whose rows therefore start on 16 bytes)
-//              take a second kernel with the same steps over 512-column
-//              tiles: four columns per thread, 16-byte copies, polarity
-//              fixed at compile time;
-//   2. scan:   one block per map counts each row segment's passing pixels
-//              (popcounts of its mask words), turns the counts into output
-//              offsets starting at the caller's *count, and advances *count;
-//   3. emit:   one warp per segment writes its detections at offset +
-//              in-segment rank, dropping (but having counted) those past
-//              capacity; segments whose count is zero cost one load.
+// Two launches for a whole batch of score maps (three when a map is very
+// tall), no atomics, so every list comes out in raster order and is identical
+// run to run:
+//   1. flags:  one warp per 2048-pixel row segment writes every pixel's
+//              pass/fail as ballot words (a bitmask in the workspace) and the
+//              segment's count.  The map streams through once; only a
+//              candidate (a score past the threshold) looks at its
+//              (2r+1)^2 window, straight from global memory, where the
+//              block's eight warps -- neighbouring rows -- have brought it
+//              into L1.  A neighbour suppresses when it comes first in the
+//              window's order (better score, or the same score at a lower
+//              linear index); out-of-frame neighbours are skipped and NaN
+//              never wins or ties, exactly like the CPU loop.
+//   2. emit:   a block takes eight segments of one map, adds up the counts of
+//              the segments before them, and each warp writes its segment's
+//              detections at offset + in-segment rank, dropping (but having
+//              counted) those past capacity.  The map's last block advances
+//              *count.  Maps of more than kDirectSegs segments, where those
+//              sums would cost more than a launch, get their offsets from a
+//              scan launch in between.
 // Semantics are the reference CPU path's (src/sam_cpu.cpp:86-138), polarity
 // included; the reference GPU kernel (src/detect.cu:43-87) ignores polarity
 // and emits in atomic arrival order, both of which this replaces.
 #include <cuda.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
@@ -37,28 +34,19 @@
 namespace hsi_b200 {
 namespace {
 
-constexpr int kThreads = 256;                // scan / emit blocks
-constexpr int kPerThread = 8;
-constexpr int kSeg = kThreads * kPerThread;  // 2048 pixels per row segment
+constexpr int kThreads = 256;
+constexpr int kWarps = kThreads / 32;        // row segments per block of flags and emit
+constexpr int kSeg = 2048;                   // pixels per row segment
 constexpr int kWordsPerSeg = kSeg / 32;      // 64
 constexpr int kMaxJobs = 64;
-// flags tiles
-constexpr int kTileW = 256;                        // columns per tile (8 ballot warps)
-constexpr int kTileH = 64;                         // rows per tile
-constexpr int kMaxRingR = 8;                       // largest radius streamed through the ring
-constexpr int kAhead = 4;                          // rows in flight ahead of the window
-constexpr int kRing = 32;                          // ring rows (a power of two >= window + spare + in flight)
-static_assert(kRing >= 2 * kMaxRingR + 2 + kAhead, "ring too small for the window");
-constexpr int kRingCols = kTileW + 2 * kMaxRingR;  // 272
-constexpr int kFlagThreads = 288;                  // >= kRingCols, whole warps
-// fast flags tiles (radius <= kFastR, width a multiple of 4)
-constexpr int kFastW = 512;                        // columns per tile, four per candidate thread
-constexpr int kFastR = 4;                          // largest radius; also the halo of a ring row
-constexpr int kFastGroups = kFastW / 4 + 2;        // float4 groups of a ring row (one halo group each side)
-constexpr int kFastAhead = 6;                      // rows in flight ahead of the window
-constexpr int kFastRing = 16;                      // ring rows
-static_assert(kFastRing >= 2 * kFastR + kFastAhead + 2, "fast ring too small for the window");
-constexpr int kFastThreads = 160;                  // >= kFastGroups, whole warps
+constexpr int kChunk = 128;                  // pixels a warp takes at a time, four per lane
+constexpr int kLaneR = 4;                    // largest radius of the lanes' own windows (one float4 group each side)
+constexpr int kFilterR = 2;                  // their radius ahead of a larger one
+// A block of emit reads the counts of all earlier segments of its map: 2 KB on
+// average for 1024 rows.  At 16384 segments (a 16384-row map) the 2048 blocks
+// read 64 MB of L2 together, about what a scan launch costs; the sums grow
+// with the square of the height.
+constexpr int kDirectSegs = 16384;
 
 struct Job {
   const float* score;
@@ -67,235 +55,185 @@ struct Job {
   float threshold;
   int radius;
   int higher;
+  int vec;           // rows start on 16 bytes
   int capacity;
   hsi_detection* out;
   uint32_t* count;
   int seg0;          // first segment of this map in the batch
   int segs_per_row;  // ceil(width / kSeg)
-  int tile0;         // first flags tile of this map among the maps of its kind
-  int tiles_x;       // ceil(width / tile width of its kind)
+  int unit0;         // first block of eight segments of this map in the batch
 };
 
+// N: job slots; a single map travels in a small parameter block.
+template <int N>
 struct Batch {
-  Job jobs[kMaxJobs];
+  Job jobs[N];
   int njobs;
-  int total_segs;
-  int kind_jobs[2][kMaxJobs];  // job indices of the plain (0) and fast (1) flags kinds, in batch order
-  int kind_n[2];
-  int kind_tiles[2];
+  int units;          // blocks of flags and of emit
   uint32_t* counts;   // [total_segs]
-  uint32_t* offsets;  // [total_segs]
+  uint32_t* offsets;  // [total_segs]; without a scan only a map's first entry: its *count at the start
   uint32_t* masks;    // [total_segs * 64]
 };
 
-__device__ __forceinline__ int find_job(const Batch& b, int seg) {
+template <int N>
+__device__ __forceinline__ int find_job(const Batch<N>& b, int unit) {
+  if constexpr (N == 1) return 0;
   int lo = 0, hi = b.njobs - 1;
   while (lo < hi) {
     const int mid = (lo + hi + 1) >> 1;
-    if (b.jobs[mid].seg0 <= seg) lo = mid; else hi = mid - 1;
+    if (b.jobs[mid].unit0 <= unit) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
 
-// Job of flags tile `tile` of kind `kind` (0 plain, 1 fast).
-__device__ __forceinline__ int find_job_tile(const Batch& b, int kind, int tile) {
-  int lo = 0, hi = b.kind_n[kind] - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (b.jobs[b.kind_jobs[kind][mid]].tile0 <= tile) lo = mid; else hi = mid - 1;
+template <bool HIGHER>
+__device__ __forceinline__ bool over_threshold(float s, float threshold) {
+  return HIGHER ? s >= threshold : s <= threshold;  // NaN fails both
+}
+
+// Whether neighbour o suppresses the candidate s: a better score, or the same
+// score when the neighbour comes `earlier` in linear index.  NaN never does.
+template <bool HIGHER>
+__device__ __forceinline__ bool suppresses(float o, float s, bool earlier) {
+  if (HIGHER) return earlier ? o >= s : o > s;
+  return earlier ? o <= s : o < s;
+}
+
+// One candidate by a whole warp, a lane per neighbour and round, rows nearest
+// the candidate first (smooth maps decide in the first round): any radius.
+// A few per cent of the pixels are candidates, so a 128-pixel chunk has two or
+// three; they cost about 20 instructions each here, where the lanes' own
+// windows (below) cost 200 to 500 for the chunk however few of its pixels are
+// candidates.  So up to kFew candidates of a chunk go one by one; more take
+// the lanes' windows, of the whole radius up to kLaneR and of kFilterR above
+// it, which leave the warp a twenty-fifth of the pixels or so.
+// 64 maps of 1024 x 1024 with 0.05, 1, 5 and 30 % of uniform random scores
+// past the threshold, radius 2: 126, 209, 375 and 394 us for both launches;
+// the ring-buffer tiles before (one barrier per row, then a scan launch) took
+// 415 to 455.  One 64 x 96 map: 5.4 us against 69, where a tile walked its 64
+// rows in one block.
+constexpr int kFew = 6;
+constexpr int kRounds = 3;  // rounds whose neighbours a lane keeps: all of them up to radius 4
+struct WarpWindow {
+  int side;              // 2 r + 1
+  int offset[kRounds];   // this lane's neighbours as linear offsets; 0 (the candidate itself) past the window
+  bool earlier[kRounds];
+};
+__device__ __forceinline__ void warp_neighbour(int k, int side, int& dx, int& dy) {
+  dx = dy = 0;
+  if (k >= static_cast<int64_t>(side) * side) return;
+  const int i = k / side;  // rows 0, 1, -1, 2, -2, ..
+  dy = (i & 1) ? (i + 1) / 2 : -(i / 2);
+  dx = k - i * side - side / 2;
+}
+__device__ __forceinline__ WarpWindow warp_window(const Job& J) {
+  WarpWindow w;
+  w.side = 2 * J.radius + 1;
+#pragma unroll
+  for (int k = 0; k < kRounds; ++k) {
+    int dx, dy;
+    warp_neighbour(32 * k + (threadIdx.x & 31), w.side, dx, dy);
+    w.offset[k] = dy * J.width + dx;
+    w.earlier[k] = dy < 0 || (dy == 0 && dx < 0);
   }
-  return b.kind_jobs[kind][lo];
+  return w;
 }
-
-__device__ __forceinline__ bool better(float a, float b, bool higher) { return higher ? a > b : a < b; }
-
-__device__ __forceinline__ bool over_threshold(float s, float threshold, bool higher) {
-  return higher ? s >= threshold : s <= threshold;  // NaN fails both
-}
-
-// Mask word of the 32 pixels of row y starting at column xw (a multiple of 32).
-__device__ __forceinline__ uint32_t* mask_word(const Batch& b, const Job& J, int y, int xw) {
-  return b.masks + static_cast<int64_t>(J.seg0 + y * J.segs_per_row + xw / kSeg) * kWordsPerSeg + (xw % kSeg) / 32;
-}
-
-__device__ __forceinline__ void cp_async4(void* dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16(void* dst, const void* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
-// NMS against global memory, for radii too large for the ring.
-__device__ bool local_best_global(const float* __restrict__ s, int x, int y, int w, int h, int r, float self,
-                                  bool higher) {
-  const int64_t self_idx = static_cast<int64_t>(y) * w + x;
-  for (int dy = -r; dy <= r; ++dy) {
-    const int ny = y + dy;
-    if (ny < 0 || ny >= h) continue;
-    for (int dx = -r; dx <= r; ++dx) {
-      if (dx == 0 && dy == 0) continue;
-      const int nx = x + dx;
-      if (nx < 0 || nx >= w) continue;
-      const int64_t n = static_cast<int64_t>(ny) * w + nx;
-      const float o = __ldg(s + n);
-      if (better(o, self, higher)) return false;
-      if (o == self && n < self_idx) return false;
+template <int R, bool HIGHER>
+__device__ __forceinline__ bool warp_suppressed(const Job& J, const WarpWindow& w, int x, int y, float s) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int r = R <= kLaneR ? R : w.side / 2;
+  constexpr int kHeld = R <= 2 ? 1 : R == 3 ? 2 : kRounds;
+  const float* p = J.score + static_cast<int64_t>(y) * J.width + x;
+  int i = 0;  // first row still to look at
+  if (x >= r && x < J.width - r && y >= r && y < J.height - r) {
+    // the whole window lies in the map; the candidate itself never suppresses
+#pragma unroll
+    for (int k = 0; k < kHeld; ++k) {
+      if (k > 0 && 32 * k >= static_cast<int64_t>(w.side) * w.side) return false;
+      if (__any_sync(kAll, suppresses<HIGHER>(__ldg(p + w.offset[k]), s, w.earlier[k]))) return true;
+    }
+    if (R <= kLaneR) return false;
+    i = 32 * kHeld / w.side;
+  }
+  // windows across the map's edge, and what is left of larger ones: row by row
+  const int lo = max(x - r, 0), hi = min(x + r, J.width - 1);
+#pragma unroll 1
+  for (; i < w.side; ++i) {
+    const int dy = (i & 1) ? (i + 1) / 2 : -(i / 2);
+    if (static_cast<unsigned>(y + dy) >= static_cast<unsigned>(J.height)) continue;
+    const float* row = p + static_cast<int64_t>(dy) * J.width - x;
+    for (int n0 = lo; n0 <= hi; n0 += 32) {
+      const int nx = n0 + (threadIdx.x & 31);
+      const bool in = nx <= hi;
+      const float o = __ldg(in ? row + nx : p);
+      if (__any_sync(kAll, suppresses<HIGHER>(o, s, in && (dy < 0 || (dy == 0 && nx < x))))) return true;
     }
   }
-  return true;
+  return false;
 }
 
-// Shared memory of one flags tile.
-struct FlagsSmem {
-  float ring[kRing][kRingCols];   // score rows, NaN outside the frame
-  float2 best[2][kRingCols];      // per column: (first-best score of the window, its row 0 .. 2r as int bits)
-  float centre[2][kRingCols];     // per column: the centre row's score
-};
+// One lane's candidate s at (x, y) against its whole window of radius R.
+template <int R, bool HIGHER>
+__device__ __forceinline__ bool lane_suppressed(const Job& J, int x, int y, float s) {
+  bool in[2 * R + 1];
+#pragma unroll
+  for (int dx = -R; dx <= R; ++dx) in[dx + R] = x + dx >= 0 && x + dx < J.width;
+  bool hit = false;
+#pragma unroll
+  for (int dy = -R; dy <= R; ++dy) {
+    if (y + dy < 0 || y + dy >= J.height) continue;
+    const float* p = J.score + static_cast<int64_t>(y + dy) * J.width + x;
+#pragma unroll
+    for (int dx = -R; dx <= R; ++dx)
+      if ((dx != 0 || dy != 0) && in[dx + R]) hit |= suppresses<HIGHER>(__ldg(p + dx), s, dy < 0 || (dy == 0 && dx < 0));
+  }
+  return hit;
+}
 
-// One tile whose window radius R is known at compile time (0 .. kMaxRingR).
-template <int R>
-__device__ __forceinline__ void flags_tile(const Batch& b, const Job& J, FlagsSmem& sm, int x0, int y0, int y1) {
-  constexpr int kCols = kTileW + 2 * R;
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+// The windows of the four pixels x .. x + 3 of a lane at a fixed radius, on
+// 16-byte groups: rows dy0 .. dy1 of the window, all of their loads in flight
+// together.  Clears the pixels of `keep` that a neighbour suppresses.  The
+// width is a multiple of 4, so a group lies wholly inside or outside the map.
+template <int R, int DY0, int DY1, bool HIGHER>
+__device__ __forceinline__ void window_rows(const Job& J, int x, int y, const float (&s)[4], unsigned& keep) {
   const float nan = __int_as_float(0x7fc00000);
-  const int W = J.width, H = J.height;
-  const bool higher = J.higher != 0;
-  const float thr = J.threshold;
-  const int cx = x0 - R + t;  // this thread's column in the vertical pass
-  const bool col_in = t < kCols && cx >= 0 && cx < W;
-  const int last = y1 - 1 + R;  // last row the tile reads
-  // One ring row per call: a 4-byte cp.async per in-frame column, NaN stored
-  // directly elsewhere, and one commit group per thread per call.
-  int next_row = y0 - R;
-  auto issue_next = [&]() {
-    if (next_row <= last && t < kCols) {
-      float* dst = &sm.ring[next_row & (kRing - 1)][t];
-      if (col_in && next_row >= 0 && next_row < H)
-        cp_async4(dst, J.score + static_cast<int64_t>(next_row) * W + cx);
-      else
-        *dst = nan;
+  float4 g[DY1 - DY0 + 1][3];
+#pragma unroll
+  for (int dy = DY0; dy <= DY1; ++dy) {
+    const int ny = y + dy;
+    const bool row = ny >= 0 && ny < J.height;
+    const float4* p = reinterpret_cast<const float4*>(J.score + static_cast<int64_t>(row ? ny : y) * J.width + x);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      const bool in = row && (k != 0 || x >= 4) && (k != 2 || x + 4 < J.width);
+      g[dy - DY0][k] = in ? __ldg(p + k - 1) : make_float4(nan, nan, nan, nan);
     }
-    cp_async_commit();
-    ++next_row;
-  };
+  }
 #pragma unroll
-  for (int k = 0; k < 2 * R + kAhead; ++k) issue_next();
-  for (int y = y0; y <= y1; ++y) {
-    // row y + R + kAhead reuses the slot of row y + R + kAhead - kRing, at
-    // most y - R - 2, whose last reader passed the previous barrier
-    if (y < y1) issue_next();
-    cp_async_wait<kAhead>();  // this thread's copies up to row y + R have landed
-    __syncthreads();          // ... and everyone's
-    if (y > y0 && t < kTileW) {
-      // candidates of row y - 1 against the column bests around them
-      const int yh = y - 1, hb = yh & 1;
-      const int x = x0 + t;
-      bool pass = false;
-      if (x < W) {
-        const float s = sm.centre[hb][t + R];
-        if (over_threshold(s, thr, higher)) {
-          pass = true;
+  for (int dy = DY0; dy <= DY1; ++dy) {
+    const float4(&q)[3] = g[dy - DY0];
+    const float v[12] = {q[0].x, q[0].y, q[0].z, q[0].w, q[1].x, q[1].y, q[1].z, q[1].w, q[2].x, q[2].y, q[2].z, q[2].w};
 #pragma unroll
-          for (int dx = -R; dx <= R; ++dx) {
-            const float2 vk = sm.best[hb][t + R + dx];
-            const float v = vk.x;
-            const int k = __float_as_int(vk.y);
-            // first in the window's order: better score, or the same score
-            // at a lower linear index (an earlier row, or this row to the left)
-            if (!isnan(v) && (better(v, s, higher) || (v == s && (k < R || (k == R && dx < 0))))) pass = false;
-          }
-        }
+    for (int j = 0; j < 4; ++j) {
+      bool hit = false;
+#pragma unroll
+      for (int dx = -R; dx <= R; ++dx) {
+        if (dy == 0 && dx == 0) continue;
+        hit |= suppresses<HIGHER>(v[4 + j + dx], s[j], dy < 0 || (dy == 0 && dx < 0));
       }
-      const uint32_t word = __ballot_sync(0xffffffffu, pass);
-      if (lane == 0 && x0 + 32 * warp < W) *mask_word(b, J, yh, x0 + 32 * warp) = word;
-    }
-    if (y < y1 && t < kCols) {
-      // column t's first-best over rows y - R .. y + R
-      float bv = nan;
-      int bk = 0;
-#pragma unroll
-      for (int k = 0; k <= 2 * R; ++k) {
-        const float v = sm.ring[(y - R + k) & (kRing - 1)][t];
-        if (!isnan(v) && (isnan(bv) || better(v, bv, higher))) {
-          bv = v;
-          bk = k;
-        }
-        if (k == R) sm.centre[y & 1][t] = v;
-      }
-      sm.best[y & 1][t] = make_float2(bv, __int_as_float(bk));
+      if (hit) keep &= ~(1u << j);
     }
   }
 }
 
-// A tile whose radius is too large for the ring: each candidate's window
-// read from global memory.
-__device__ void flags_tile_global(const Batch& b, const Job& J, int x0, int y0, int y1) {
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
-  const int r = J.radius;
-  const bool higher = J.higher != 0;
-  for (int y = y0; y < y1; ++y) {
-    if (t >= kTileW) continue;
-    const int x = x0 + t;
-    bool pass = false;
-    if (x < J.width) {
-      const float s = J.score[static_cast<int64_t>(y) * J.width + x];
-      pass = over_threshold(s, J.threshold, higher) &&
-             local_best_global(J.score, x, y, J.width, J.height, r, s, higher);
-    }
-    const uint32_t word = __ballot_sync(0xffffffffu, pass);
-    if (lane == 0 && x0 + 32 * warp < J.width) *mask_word(b, J, y, x0 + 32 * warp) = word;
-  }
-}
-
-__global__ void __launch_bounds__(kFlagThreads) flags_kernel(const __grid_constant__ Batch b) {
-  __shared__ FlagsSmem sm;
-  for (int tile = blockIdx.x; tile < b.kind_tiles[0]; tile += gridDim.x) {
-    __syncthreads();  // the previous tile is done with the shared buffers
-    const Job& J = b.jobs[find_job_tile(b, 0, tile)];
-    const int local = tile - J.tile0;
-    const int x0 = (local % J.tiles_x) * kTileW;
-    const int y0 = (local / J.tiles_x) * kTileH;
-    const int y1 = min(J.height, y0 + kTileH);
-    switch (J.radius > 0 ? J.radius : 0) {
-      case 0: flags_tile<0>(b, J, sm, x0, y0, y1); break;
-      case 1: flags_tile<1>(b, J, sm, x0, y0, y1); break;
-      case 2: flags_tile<2>(b, J, sm, x0, y0, y1); break;
-      case 3: flags_tile<3>(b, J, sm, x0, y0, y1); break;
-      case 4: flags_tile<4>(b, J, sm, x0, y0, y1); break;
-      case 5: flags_tile<5>(b, J, sm, x0, y0, y1); break;
-      case 6: flags_tile<6>(b, J, sm, x0, y0, y1); break;
-      case 7: flags_tile<7>(b, J, sm, x0, y0, y1); break;
-      case 8: flags_tile<8>(b, J, sm, x0, y0, y1); break;
-      default: flags_tile_global(b, J, x0, y0, y1); break;
-    }
-  }
-}
-
-// Shared memory of one fast flags tile: ring rows as float4 groups starting
-// kFastR columns left of the tile, and per group the column bests of the
-// window (score, row 0 .. 2r) for two consecutive rows.
-struct FastSmem {
-  float4 ring[kFastRing][kFastGroups];
-  float4 bv[2][kFastGroups];
-  int4 bk[2][kFastGroups];
-};
-
-template <bool HIGHER>
-__device__ __forceinline__ bool better_t(float a, float b) { return HIGHER ? a > b : a < b; }
-
-// Column c's first-best update with the value v of window row k (NaN never
-// wins; the first non-NaN value always does).
-template <bool HIGHER>
-__device__ __forceinline__ void best_update(float v, int k, float& bv, int& bk) {
-  if (!isnan(v) && (isnan(bv) || better_t<HIGHER>(v, bv))) {
-    bv = v;
-    bk = k;
-  }
+// Three rows at a time: 36 registers of loads in flight.
+template <int R, bool HIGHER, int DY = -R>
+__device__ __forceinline__ void window(const Job& J, int x, int y, const float (&s)[4], unsigned& keep) {
+  static_assert(R >= 1 && R <= kLaneR, "one group each side");
+  if (keep == 0) return;
+  constexpr int kLast = DY + 2 < R ? DY + 2 : R;
+  window_rows<R, DY, kLast, HIGHER>(J, x, y, s, keep);
+  if constexpr (kLast < R) window<R, HIGHER, kLast + 1>(J, x, y, s, keep);
 }
 
 // Bits 0..7 of x moved to bits 0, 4, .., 28.
@@ -306,171 +244,161 @@ __device__ __forceinline__ uint32_t spread4(uint32_t x) {
   return x;
 }
 
-// One fast tile: the steps of flags_tile with four adjacent columns per
-// thread.  Thread g < kFastGroups copies and reduces ring group g (columns
-// x0 - kFastR + 4g ..); thread t < kFastW / 4 tests columns x0 + 4t .. + 3,
-// whose windows lie in groups t .. t + 2.  The width is a multiple of 4, so
-// a group lies wholly inside or wholly outside the frame.
-template <int R, bool HIGHER>
-__device__ __forceinline__ void flags_fast_tile(const Batch& b, const Job& J, FastSmem& sm, int x0, int y0, int y1) {
-  static_assert(R <= kFastR, "radius above the fast halo");
-  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+// The four pixels of a lane in one chunk.  VEC (rows on 16 bytes, width a
+// multiple of 4): columns 4l .. 4l + 3; otherwise l, l + 32, l + 64, l + 96.
+template <bool VEC>
+__device__ __forceinline__ int column_of(int lane, int j) { return VEC ? 4 * lane + j : 32 * j + lane; }
+
+template <bool VEC>
+__device__ __forceinline__ float4 load_chunk(const float* __restrict__ row, int x0, int end) {
+  const int lane = threadIdx.x & 31;
   const float nan = __int_as_float(0x7fc00000);
-  const float4 nan4 = make_float4(nan, nan, nan, nan);
-  const int W = J.width, H = J.height;
-  const float thr = J.threshold;
-  const bool loader = t < kFastGroups;
-  const int gx = x0 - kFastR + 4 * t;  // first column of this thread's group
-  const bool col_in = loader && gx >= 0 && gx < W;
-  const int last = y1 - 1 + R;  // last row the tile reads
-  int next_row = y0 - R;
-  auto issue_next = [&]() {
-    if (next_row <= last && loader) {
-      float4* dst = &sm.ring[next_row & (kFastRing - 1)][t];
-      if (col_in && next_row >= 0 && next_row < H)
-        cp_async16(dst, J.score + static_cast<int64_t>(next_row) * W + gx);
-      else
-        *dst = nan4;
-    }
-    cp_async_commit();
-    ++next_row;
-  };
+  float4 c = make_float4(nan, nan, nan, nan);
+  if constexpr (VEC) {
+    if (x0 + 4 * lane < end) c = __ldg(reinterpret_cast<const float4*>(row + x0 + 4 * lane));
+  } else {
+    const float* p = row + x0 + lane;
+    if (x0 + lane < end) c.x = __ldg(p);
+    if (x0 + lane + 32 < end) c.y = __ldg(p + 32);
+    if (x0 + lane + 64 < end) c.z = __ldg(p + 64);
+    if (x0 + lane + 96 < end) c.w = __ldg(p + 96);
+  }
+  return c;
+}
+
+// One segment: mask words and count.  R = kLaneR + 1 stands for any radius
+// above kLaneR.  The body of a chunk exists once per instance (the candidates
+// of all four pixel slots share one loop, three chunks are loaded ahead by
+// rotation instead of unrolling): unrolled sixteen-fold the instances
+// outgrew the instruction cache and ran at half this speed.
+template <int R, bool HIGHER, bool VEC>
+__device__ __forceinline__ uint32_t flag_segment(const Job& J, int y, int xs, uint32_t* mask) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const int end = min(J.width, xs + kSeg);
+  const float* row = J.score + static_cast<int64_t>(y) * J.width;
+  uint32_t total = 0;
+  WarpWindow ww{};
+  if constexpr (R > 0) ww = warp_window(J);
+  float4 c = load_chunk<VEC>(row, xs, end), c1 = load_chunk<VEC>(row, xs + kChunk, end);
+  float4 c2 = load_chunk<VEC>(row, xs + 2 * kChunk, end);
+#pragma unroll 1
+  for (int xc = xs; xc < end; xc += kChunk) {
+    const float4 c3 = load_chunk<VEC>(row, xc + 3 * kChunk, end);
+    const float s[4] = {c.x, c.y, c.z, c.w};
+    unsigned keep = 0;  // bit j: pixel j of this lane passes
 #pragma unroll
-  for (int k = 0; k < 2 * R + kFastAhead; ++k) issue_next();
-  for (int y = y0; y <= y1; ++y) {
-    // row y + R + kFastAhead reuses the slot of row y + R + kFastAhead -
-    // kFastRing <= y - R - 2; the rows still read are y - 1 - R and later
-    if (y < y1) issue_next();
-    cp_async_wait<kFastAhead>();  // this thread's copies up to row y + R have landed
-    __syncthreads();              // ... and everyone's
-    if (y > y0 && t < kFastW / 4) {
-      // candidates of row y - 1 (its scores are still in the ring) against
-      // the column bests around them
-      const int yh = y - 1, hb = yh & 1;
-      const float4 c4 = sm.ring[yh & (kFastRing - 1)][t + 1];
-      const float s[4] = {c4.x, c4.y, c4.z, c4.w};
-      float v[12];
-      int k[12];
-#pragma unroll
-      for (int g = 0; g < 3; ++g) {
-        const float4 a = sm.bv[hb][t + g];
-        const int4 q = sm.bk[hb][t + g];
-        v[4 * g] = a.x; v[4 * g + 1] = a.y; v[4 * g + 2] = a.z; v[4 * g + 3] = a.w;
-        k[4 * g] = q.x; k[4 * g + 1] = q.y; k[4 * g + 2] = q.z; k[4 * g + 3] = q.w;
-      }
-      const bool in = x0 + 4 * t < W;
-      uint32_t word[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        bool pass = in && (HIGHER ? s[j] >= thr : s[j] <= thr);  // NaN fails both
-#pragma unroll
-        for (int dx = -R; dx <= R; ++dx) {
-          const int o = kFastR + j + dx;
-          // first in the window's order: better score, or the same score at
-          // a lower linear index (an earlier row, or this row to the left)
-          const bool earlier = dx < 0 ? k[o] <= R : k[o] < R;
-          if (better_t<HIGHER>(v[o], s[j]) || (v[o] == s[j] && earlier)) pass = false;
+    for (int j = 0; j < 4; ++j) keep |= over_threshold<HIGHER>(s[j], J.threshold) ? 1u << j : 0u;
+    if constexpr (R > 0) {
+      unsigned n = __reduce_add_sync(kAll, __popc(keep));
+      if (n > kFew) {
+        constexpr int kR = R <= kLaneR ? R : kFilterR;
+        if constexpr (VEC) {
+          window<kR, HIGHER>(J, xc + 4 * lane, y, s, keep);
+        } else {
+#pragma unroll 1
+          for (int j = 0; j < 4; ++j) {
+            const float sj = j < 2 ? (j == 0 ? s[0] : s[1]) : (j == 2 ? s[2] : s[3]);
+            if (((keep >> j) & 1u) && lane_suppressed<kR, HIGHER>(J, xc + column_of<VEC>(lane, j), y, sj))
+              keep &= ~(1u << j);
+          }
         }
-        word[j] = __ballot_sync(0xffffffffu, pass);  // bit l: column 4l + j of the warp's 128
+        __syncwarp();
+        if constexpr (R <= kLaneR) n = 0;  // decided
       }
-      if (lane < 4) {
-        // mask word `lane` of the warp: its columns 32 lane + 4i + j come
-        // from bit 8 lane + i of word[j]
-        uint32_t m = 0u;
+      if (n > 0) {
+        unsigned todo = keep;
+        for (unsigned lanes = __ballot_sync(kAll, todo != 0u); lanes != 0u; lanes = __ballot_sync(kAll, todo != 0u)) {
+          const int l = __ffs(lanes) - 1;
+          const int j = __ffs(__shfl_sync(kAll, todo, l)) - 1;
+          const float mine = j < 2 ? (j == 0 ? s[0] : s[1]) : (j == 2 ? s[2] : s[3]);
+          const float sl = __shfl_sync(kAll, mine, l);
+          const bool out = warp_suppressed<R, HIGHER>(J, ww, xc + column_of<VEC>(l, j), y, sl);
+          if (lane == l) {
+            todo &= todo - 1u;
+            if (out) keep &= ~(1u << j);
+          }
+        }
+      }
+    }
+    uint32_t word[4];  // bit l of word j: column_of(l, j)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) total += __popc(word[j] = __ballot_sync(kAll, (keep >> j) & 1u));
+    if (lane < 4 && xc + 32 * lane < end) {
+      uint32_t m = 0u;
+      if constexpr (VEC) {  // columns 32 lane + 4i + j come from bit 8 lane + i of word[j]
 #pragma unroll
         for (int j = 0; j < 4; ++j) m |= spread4((word[j] >> (8 * lane)) & 0xffu) << j;
-        const int xw = x0 + 128 * warp + 32 * lane;
-        if (xw < W) *mask_word(b, J, yh, xw) = m;
+      } else {
+        m = lane < 2 ? (lane == 0 ? word[0] : word[1]) : (lane == 2 ? word[2] : word[3]);
       }
+      mask[(xc - xs) / 32 + lane] = m;
     }
-    if (y < y1 && loader) {
-      // group t's column first-bests over rows y - R .. y + R
-      float4 bv = nan4;
-      int4 bk = make_int4(0, 0, 0, 0);
-#pragma unroll
-      for (int k = 0; k <= 2 * R; ++k) {
-        const float4 a = sm.ring[(y - R + k) & (kFastRing - 1)][t];
-        best_update<HIGHER>(a.x, k, bv.x, bk.x);
-        best_update<HIGHER>(a.y, k, bv.y, bk.y);
-        best_update<HIGHER>(a.z, k, bv.z, bk.z);
-        best_update<HIGHER>(a.w, k, bv.w, bk.w);
-      }
-      sm.bv[y & 1][t] = bv;
-      sm.bk[y & 1][t] = bk;
-    }
+    c = c1;
+    c1 = c2;
+    c2 = c3;
   }
+  return total;
+}
+
+template <int R, bool HIGHER>
+__device__ __forceinline__ uint32_t flag_radius(const Job& J, int y, int xs, uint32_t* mask) {
+  return J.vec ? flag_segment<R, HIGHER, true>(J, y, xs, mask) : flag_segment<R, HIGHER, false>(J, y, xs, mask);
 }
 
 template <bool HIGHER>
-__device__ __forceinline__ void flags_fast_dispatch(const Batch& b, const Job& J, FastSmem& sm, int x0, int y0,
-                                                    int y1) {
+__device__ __forceinline__ uint32_t flag_dispatch(const Job& J, int y, int xs, uint32_t* mask) {
   switch (J.radius > 0 ? J.radius : 0) {
-    case 0: flags_fast_tile<0, HIGHER>(b, J, sm, x0, y0, y1); break;
-    case 1: flags_fast_tile<1, HIGHER>(b, J, sm, x0, y0, y1); break;
-    case 2: flags_fast_tile<2, HIGHER>(b, J, sm, x0, y0, y1); break;
-    case 3: flags_fast_tile<3, HIGHER>(b, J, sm, x0, y0, y1); break;
-    default: flags_fast_tile<4, HIGHER>(b, J, sm, x0, y0, y1); break;  // the host admits radius <= kFastR only
+    case 0: return flag_radius<0, HIGHER>(J, y, xs, mask);
+    case 1: return flag_radius<1, HIGHER>(J, y, xs, mask);
+    case 2: return flag_radius<2, HIGHER>(J, y, xs, mask);
+    case 3: return flag_radius<3, HIGHER>(J, y, xs, mask);
+    case 4: return flag_radius<4, HIGHER>(J, y, xs, mask);
+    default: return flag_radius<kLaneR + 1, HIGHER>(J, y, xs, mask);
   }
 }
 
-__global__ void __launch_bounds__(kFastThreads) flags_fast_kernel(const __grid_constant__ Batch b) {
-  __shared__ FastSmem sm;
-  for (int tile = blockIdx.x; tile < b.kind_tiles[1]; tile += gridDim.x) {
-    __syncthreads();  // the previous tile is done with the shared buffers
-    const Job& J = b.jobs[find_job_tile(b, 1, tile)];
-    const int local = tile - J.tile0;
-    const int x0 = (local % J.tiles_x) * kFastW;
-    const int y0 = (local / J.tiles_x) * kTileH;
-    const int y1 = min(J.height, y0 + kTileH);
-    if (J.higher)
-      flags_fast_dispatch<true>(b, J, sm, x0, y0, y1);
-    else
-      flags_fast_dispatch<false>(b, J, sm, x0, y0, y1);
+template <int N>
+__global__ void __launch_bounds__(kThreads, 4) flags_kernel(const __grid_constant__ Batch<N> b) {
+  const Job& J = b.jobs[find_job(b, blockIdx.x)];
+  const int local = (blockIdx.x - J.unit0) * kWarps + (threadIdx.x >> 5);
+  if (local >= J.height * J.segs_per_row) return;
+  const int y = local / J.segs_per_row, xs = (local % J.segs_per_row) * kSeg;
+  const int seg = J.seg0 + local;
+  uint32_t* mask = b.masks + static_cast<int64_t>(seg) * kWordsPerSeg;
+  const uint32_t n = J.higher ? flag_dispatch<true>(J, y, xs, mask) : flag_dispatch<false>(J, y, xs, mask);
+  if ((threadIdx.x & 31) == 0) {
+    b.counts[seg] = n;
+    if (local == 0) b.offsets[seg] = *J.count;  // before emit's last block advances it
   }
 }
 
-// Passing pixels of segment `seg` of job J: popcount of its mask words that
-// cover pixels of the map (words past the row's end are never written).
+// Mask words of segment `local` of job J that cover pixels of the map (words
+// past the row's end are never written).
 __device__ __forceinline__ int seg_words(const Job& J, int local) {
   const int xs = (local % J.segs_per_row) * kSeg;
   const int len = min(kSeg, J.width - xs);
   return (len + 31) / 32;
 }
 
-// One block per map: segment counts from the masks, their exclusive scan from
-// *count; *count += total.
-__global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ Batch b) {
+// One block per map: the segments' offsets, from *count; *count += total.
+template <int N>
+__global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ Batch<N> b) {
   __shared__ uint32_t s_warp[32];
-  __shared__ uint32_t s_carry;
   const Job& J = b.jobs[blockIdx.x];
   const int segs = J.height * J.segs_per_row;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) s_carry = *J.count;
-  __syncthreads();
+  uint32_t carry = *J.count;
   for (int chunk = 0; chunk < segs; chunk += 1024) {
-    // warp w counts segments chunk + 32 w .. + 31, one per step; lane k
-    // keeps the count of segment chunk + 32 w + k (= this thread's)
-    uint32_t v = 0u;
-    for (int k = 0; k < 32; ++k) {
-      const int si = chunk + warp * 32 + k;
-      uint32_t c = 0u;
-      if (si < segs) {
-        const int nw = seg_words(J, si);
-        const uint32_t* m = b.masks + static_cast<int64_t>(J.seg0 + si) * kWordsPerSeg;
-        c = (lane < nw ? __popc(m[lane]) : 0) + (lane + 32 < nw ? __popc(m[lane + 32]) : 0);
-      }
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
-      if (lane == k) v = c;
-    }
     const int i = chunk + threadIdx.x;
-    if (i < segs) b.counts[J.seg0 + i] = v;
+    const uint32_t v = i < segs ? b.counts[J.seg0 + i] : 0u;
     uint32_t incl = v;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
       const uint32_t o = __shfl_up_sync(0xffffffffu, incl, d);
       if (lane >= d) incl += o;
     }
+    __syncthreads();  // the previous chunk's sums have been read
     if (lane == 31) s_warp[warp] = incl;
     __syncthreads();
     if (warp == 0) {
@@ -483,70 +411,96 @@ __global__ void __launch_bounds__(1024) scan_kernel(const __grid_constant__ Batc
       s_warp[lane] = w;
     }
     __syncthreads();
-    const uint32_t warp_base = warp > 0 ? s_warp[warp - 1] : 0u;
-    const uint32_t carry = s_carry;
-    if (i < segs) b.offsets[J.seg0 + i] = carry + warp_base + incl - v;
-    __syncthreads();
-    if (threadIdx.x == 0) s_carry = carry + s_warp[31];
-    __syncthreads();
+    if (i < segs) b.offsets[J.seg0 + i] = carry + (warp > 0 ? s_warp[warp - 1] : 0u) + incl - v;
+    carry += s_warp[31];
   }
-  if (threadIdx.x == 0) *J.count = s_carry;
+  __syncthreads();  // every thread has read *count
+  if (threadIdx.x == 0) *J.count = carry;
 }
 
-// One warp per segment.  Lane l holds mask words l and l + 32, their
-// exclusive prefix of popcounts comes from two shuffle scans, and the warp
-// then visits the non-empty words in order with lane = bit, so that the
-// detections of one word go to consecutive slots in one coalesced store.
-__global__ void __launch_bounds__(kThreads) emit_kernel(const __grid_constant__ Batch b) {
-  const int lane = threadIdx.x & 31;
-  const int warps = gridDim.x * (kThreads / 32);
-  const uint32_t lt = (1u << lane) - 1u;
-  for (int seg = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5); seg < b.total_segs; seg += warps) {
-    const uint32_t count = b.counts[seg];
-    if (count == 0u) continue;  // nothing passed in this segment (the same for the whole warp)
-    const Job& J = b.jobs[find_job(b, seg)];
-    const int local = seg - J.seg0;
-    const int nw = seg_words(J, local);
-    const uint32_t* m = b.masks + static_cast<int64_t>(seg) * kWordsPerSeg;
-    const uint32_t w0 = lane < nw ? m[lane] : 0u;
-    const uint32_t w1 = lane + 32 < nw ? m[lane + 32] : 0u;
-    const uint32_t base = b.offsets[seg];
-    const uint32_t c0 = __popc(w0), c1 = __popc(w1);
-    uint32_t i0 = c0, i1 = c1;  // inclusive scans over the lanes
+// One warp per segment, eight consecutive segments of a map per block.  Lane l
+// holds mask words l and l + 32, their exclusive prefix of popcounts comes
+// from two shuffle scans, and the warp then visits the non-empty words in
+// order with lane = bit, so that the detections of one word go to consecutive
+// slots in one coalesced store.
+template <int N, bool SCANNED>
+__global__ void __launch_bounds__(kThreads) emit_kernel(const __grid_constant__ Batch<N> b) {
+  __shared__ uint32_t s_sum[kWarps];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const Job& J = b.jobs[find_job(b, blockIdx.x)];
+  const int segs = J.height * J.segs_per_row;
+  const int first = (blockIdx.x - J.unit0) * kWarps;  // this block's segments
+  const int local = first + warp;
+  const int seg = J.seg0 + local;
+  const uint32_t* counts = b.counts + J.seg0;
+  const uint32_t count = local < segs ? counts[local] : 0u;
+  uint32_t base;
+  if constexpr (SCANNED) {
+    if (count == 0u) return;  // nothing passed in this segment (the same for the whole warp)
+    base = b.offsets[seg];
+  } else {
+    const bool last = first + kWarps >= segs;
+    if (!__syncthreads_or(count != 0u) && !last) return;
+    uint32_t before = 0;
+#pragma unroll 4
+    for (int i = threadIdx.x; i < first; i += kThreads) before += counts[i];
+    before = __reduce_add_sync(0xffffffffu, before);
+    if (lane == 0) s_sum[warp] = before;
+    __syncthreads();
+    base = b.offsets[J.seg0];
 #pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-      const uint32_t o0 = __shfl_up_sync(0xffffffffu, i0, d);
-      const uint32_t o1 = __shfl_up_sync(0xffffffffu, i1, d);
-      if (lane >= d) {
-        i0 += o0;
-        i1 += o1;
-      }
+    for (int w = 0; w < kWarps; ++w) base += s_sum[w];
+    uint32_t mine = 0, all = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) {
+      const uint32_t c = first + w < segs ? counts[first + w] : 0u;
+      if (w < warp) mine += c;
+      all += c;
     }
-    const uint32_t first_half = __shfl_sync(0xffffffffu, i0, 31);
-    const uint32_t e0 = i0 - c0, e1 = first_half + i1 - c1;  // exclusive prefixes of words lane, lane + 32
-    const int y = local / J.segs_per_row;
-    const int x0 = (local % J.segs_per_row) * kSeg;
+    if (last && threadIdx.x == 0) *J.count = base + all;
+    base += mine;
+    if (count == 0u) return;
+  }
+  const uint32_t lt = (1u << lane) - 1u;
+  const int nw = seg_words(J, local);
+  const uint32_t* m = b.masks + static_cast<int64_t>(seg) * kWordsPerSeg;
+  const uint32_t w0 = lane < nw ? m[lane] : 0u;
+  const uint32_t w1 = lane + 32 < nw ? m[lane + 32] : 0u;
+  const uint32_t c0 = __popc(w0), c1 = __popc(w1);
+  uint32_t i0 = c0, i1 = c1;  // inclusive scans over the lanes
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const uint32_t mine = half ? w1 : w0, pre = half ? e1 : e0;
-      uint32_t nonempty = __ballot_sync(0xffffffffu, mine != 0u);
-      while (nonempty) {
-        const int wi = __ffs(nonempty) - 1;
-        nonempty &= nonempty - 1u;
-        const uint32_t word = __shfl_sync(0xffffffffu, mine, wi);
-        const uint32_t wpre = __shfl_sync(0xffffffffu, pre, wi);
-        if ((word >> lane) & 1u) {
-          const uint32_t slot = base + wpre + __popc(word & lt);
-          if (slot < static_cast<uint32_t>(J.capacity)) {
-            const int x = x0 + (32 * half + wi) * 32 + lane;
-            const int64_t p = static_cast<int64_t>(y) * J.width + x;
-            hsi_detection d;
-            d.x = x;
-            d.y = y;
-            d.target = J.target ? J.target[p] : 0;
-            d.score = J.score[p];
-            J.out[slot] = d;
-          }
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t o0 = __shfl_up_sync(0xffffffffu, i0, d);
+    const uint32_t o1 = __shfl_up_sync(0xffffffffu, i1, d);
+    if (lane >= d) {
+      i0 += o0;
+      i1 += o1;
+    }
+  }
+  const uint32_t first_half = __shfl_sync(0xffffffffu, i0, 31);
+  const uint32_t e0 = i0 - c0, e1 = first_half + i1 - c1;  // exclusive prefixes of words lane, lane + 32
+  const int y = local / J.segs_per_row;
+  const int x0 = (local % J.segs_per_row) * kSeg;
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const uint32_t mine = half ? w1 : w0, pre = half ? e1 : e0;
+    uint32_t nonempty = __ballot_sync(0xffffffffu, mine != 0u);
+    while (nonempty) {
+      const int wi = __ffs(nonempty) - 1;
+      nonempty &= nonempty - 1u;
+      const uint32_t word = __shfl_sync(0xffffffffu, mine, wi);
+      const uint32_t wpre = __shfl_sync(0xffffffffu, pre, wi);
+      if ((word >> lane) & 1u) {
+        const uint32_t slot = base + wpre + __popc(word & lt);
+        if (slot < static_cast<uint32_t>(J.capacity)) {
+          const int x = x0 + (32 * half + wi) * 32 + lane;
+          const int64_t p = static_cast<int64_t>(y) * J.width + x;
+          hsi_detection d;
+          d.x = x;
+          d.y = y;
+          d.target = J.target ? J.target[p] : 0;
+          d.score = J.score[p];
+          J.out[slot] = d;
         }
       }
     }
@@ -563,20 +517,11 @@ constexpr int64_t kMaxBatchSegs = 0x3fffffff;
 
 size_t ws_bytes_for_segs(int64_t segs) { return static_cast<size_t>(segs) * sizeof(uint32_t) * (2 + kWordsPerSeg) + 256; }
 
-int sm_count() { return device_sm_count(); }
-
-// Blocks of `kernel` resident per SM of the current device at `threads`
-// threads (4 if the query fails).
-template <typename K>
-int resident_blocks(K* kernel, int threads) {
-  const int v = device_residency(kernel, threads, 0);
-  return v > 0 ? v : 4;
-}
-
-int run_batch(const hsi_detect_job* jobs, int n, void* ws, size_t ws_bytes, cudaStream_t s) {
-  if (!jobs || n <= 0 || n > kMaxJobs) return HSI_E_INVALID;
-  Batch b{};
-  int64_t segs = 0, tiles[2] = {0, 0};
+template <int N>
+int launch_batch(const hsi_detect_job* jobs, int n, void* ws, size_t ws_bytes, cudaStream_t s) {
+  Batch<N> b;
+  int64_t segs = 0, units = 0;
+  bool direct = true;
   for (int i = 0; i < n; ++i) {
     const hsi_detect_job& j = jobs[i];
     if (!j.score || !j.count || j.height <= 0 || j.width <= 0 || j.capacity < 0) return HSI_E_INVALID;
@@ -588,52 +533,43 @@ int run_batch(const hsi_detect_job* jobs, int n, void* ws, size_t ws_bytes, cuda
     J.height = j.height;
     J.width = j.width;
     J.threshold = j.threshold;
-    J.radius = j.nms_radius;
+    // a window past the map's far edges sees no more of it
+    J.radius = std::min(j.nms_radius, std::max(j.height, j.width));
     J.higher = j.polarity == HSI_HIGHER_IS_BETTER;
+    J.vec = j.width % 4 == 0 && (reinterpret_cast<uintptr_t>(j.score) & 15u) == 0;
     J.capacity = j.capacity;
     J.out = j.out;
     J.count = j.count;
     J.seg0 = static_cast<int>(segs);
     J.segs_per_row = (j.width + kSeg - 1) / kSeg;
-    // fast flags tiles: radius <= kFastR and rows that start on 16 bytes
-    const int kind = j.nms_radius <= kFastR && j.width % 4 == 0 &&
-                     (reinterpret_cast<uintptr_t>(j.score) & 15u) == 0;
-    const int tile_w = kind ? kFastW : kTileW;
-    J.tile0 = static_cast<int>(tiles[kind]);
-    J.tiles_x = (j.width + tile_w - 1) / tile_w;
-    b.kind_jobs[kind][b.kind_n[kind]++] = i;
-    segs += segs_of(j.height, j.width);
-    tiles[kind] += static_cast<int64_t>(J.tiles_x) * ((j.height + kTileH - 1) / kTileH);
-    if (segs > kMaxBatchSegs || tiles[kind] > 0x3fffffff) return HSI_E_CAPACITY;
+    J.unit0 = static_cast<int>(units);
+    const int64_t map_segs = segs_of(j.height, j.width);
+    segs += map_segs;
+    units += (map_segs + kWarps - 1) / kWarps;
+    if (segs > kMaxBatchSegs) return HSI_E_CAPACITY;
+    direct = direct && map_segs <= kDirectSegs;
   }
   if (!ws || ws_bytes < ws_bytes_for_segs(segs)) return HSI_E_WORKSPACE;
   if ((reinterpret_cast<uintptr_t>(ws) & 15u) != 0) return HSI_E_INVALID;
   b.njobs = n;
-  b.total_segs = static_cast<int>(segs);
-  b.kind_tiles[0] = static_cast<int>(tiles[0]);
-  b.kind_tiles[1] = static_cast<int>(tiles[1]);
+  b.units = static_cast<int>(units);
   uint32_t* p = static_cast<uint32_t*>(ws);
   b.counts = p;
   b.offsets = p + segs;
   b.masks = p + 2 * segs;
-  // one wave of resident tiles per flags kind (41 KB of shared memory each),
-  // the residency read once per device
-  const int per_sm[2] = {resident_blocks(flags_kernel, kFlagThreads),
-                         resident_blocks(flags_fast_kernel, kFastThreads)};
-  const int64_t emit_blocks = (segs + kThreads / 32 - 1) / (kThreads / 32);  // a warp per segment
-  const int grid = static_cast<int>(emit_blocks < 16 * sm_count() ? emit_blocks : 16 * sm_count());
-  for (int kind = 0; kind < 2; ++kind) {
-    if (tiles[kind] == 0) continue;
-    const int64_t wave = static_cast<int64_t>(per_sm[kind]) * sm_count();
-    const int flag_grid = static_cast<int>(tiles[kind] < wave ? tiles[kind] : wave);
-    if (kind == 0)
-      flags_kernel<<<flag_grid, kFlagThreads, 0, s>>>(b);
-    else
-      flags_fast_kernel<<<flag_grid, kFastThreads, 0, s>>>(b);
+  flags_kernel<N><<<b.units, kThreads, 0, s>>>(b);
+  if (direct) {
+    emit_kernel<N, false><<<b.units, kThreads, 0, s>>>(b);
+  } else {
+    scan_kernel<N><<<n, 1024, 0, s>>>(b);
+    emit_kernel<N, true><<<b.units, kThreads, 0, s>>>(b);
   }
-  scan_kernel<<<n, 1024, 0, s>>>(b);
-  emit_kernel<<<grid, kThreads, 0, s>>>(b);
   return static_cast<int>(cudaGetLastError());
+}
+
+int run_batch(const hsi_detect_job* jobs, int n, void* ws, size_t ws_bytes, cudaStream_t s) {
+  if (!jobs || n <= 0 || n > kMaxJobs) return HSI_E_INVALID;
+  return n == 1 ? launch_batch<1>(jobs, n, ws, ws_bytes, s) : launch_batch<kMaxJobs>(jobs, n, ws, ws_bytes, s);
 }
 
 }  // namespace
@@ -686,7 +622,7 @@ extern "C" HSI_API int hsi_detect_batch(const hsi_detect_job* jobs, int num_jobs
 // For callers that cannot allocate device memory at all -- for example a
 // plug-in that a host application hands only its input and output buffers,
 // while the application owns every byte of device memory and lets nothing
-// else call cudaMalloc -- hsi_detect_noalloc runs the same three launches as
+// else call cudaMalloc -- hsi_detect_noalloc runs the same launches as
 // hsi_detect with its scratch in the file-scope array below instead of a
 // caller workspace.  The array is part of the library's device image, so
 // every GPU that loads the library holds it (2.06 MiB) until the process

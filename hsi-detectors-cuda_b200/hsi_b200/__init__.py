@@ -336,7 +336,7 @@ def detect_batch_workspace_bytes(jobs) -> int:
 
 
 def detect_batch(jobs, workspace, stream=None) -> None:
-    """Up to 64 maps in three launches; see hsi_detect_batch."""
+    """Up to 64 maps in two launches; see hsi_detect_batch."""
     arr = (DetectJob * len(jobs))(*jobs)
     check(lib().hsi_detect_batch(arr, len(jobs), _ptr(workspace), workspace.numel(), _stream(stream)),
           "hsi_detect_batch")

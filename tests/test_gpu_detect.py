@@ -182,3 +182,42 @@ def test_unaligned_map_takes_the_plain_kernel(hsi, orc):
         n, got = hsi.detections_to_numpy(cnt, out, 1 << 16)
         assert n == n0
         assert _tuples(got) == _tuples(want)
+
+
+@pytest.mark.parametrize("shape", [(16387, 5), (16400, 8), (8193, 2052)])
+@pytest.mark.parametrize("radius", [0, 2, 4, 5])
+def test_tall_maps_bit_exact(hsi, orc, shape, radius):
+    """Maps above the segment count up to which the emitting blocks add up the counts
+    themselves (16384 segments; the last shape has two segments per row), appended
+    after entries that are already in the list."""
+    H, W = shape
+    rng = np.random.default_rng(H + W + radius)
+    score = (rng.integers(0, 400, H * W) / 400.0).astype(np.float32)
+    n0, want = orc.detect(score, None, H, W, 0.02, radius, False, capacity=1 << 22)
+    s = torch.from_numpy(score).cuda()
+    count = torch.full((1,), 3, dtype=torch.int32, device="cuda")
+    cap = n0 + 8
+    count, out = hsi.detect(s, None, H, W, 0.02, radius, 0, cap, count=count)
+    torch.cuda.synchronize()
+    assert int(count.item()) == n0 + 3
+    dt = np.dtype([("x", "<i4"), ("y", "<i4"), ("target", "<i4"), ("score", "<f4")])
+    assert out[3:3 + n0].cpu().numpy().copy().view(dt).reshape(-1).tolist() == want.tolist()
+
+
+@pytest.mark.parametrize("shape", [(40, 516), (40, 517), (1, 30000), (70, 33)])
+@pytest.mark.parametrize("radius", [1, 2, 3, 4, 6, 40, 1 << 30])
+@pytest.mark.parametrize("share", [0.01, 0.2, 1.0])
+def test_candidate_densities_bit_exact(hsi, orc, shape, radius, share):
+    """Few candidates (each taken by a whole warp), many (cut down by the lanes' own
+    windows first) and every pixel, at the map's edges and inside, with ties and NaN."""
+    H, W = shape
+    if radius == 1 << 30 and share == 1.0:
+        share = 0.05
+    rng = np.random.default_rng(H + W + radius % 1000)
+    score = (rng.integers(0, 300, H * W) / 300.0).astype(np.float32)
+    score[rng.integers(0, H * W, 5)] = np.nan
+    reach = min(radius, max(H, W))  # the oracle walks the whole window
+    n0, want = orc.detect(score, None, H, W, share, reach, False, capacity=1 << 20)
+    n, got = _gpu_detect(hsi, score, None, H, W, share, radius, False)
+    assert n == n0
+    assert _tuples(got) == _tuples(want)

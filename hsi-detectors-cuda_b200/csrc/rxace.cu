@@ -13,59 +13,118 @@
 // Waug = [W ; V^T] ((B + T) x B): the first B rows give z, the last T rows the
 // ACE numerators, and an epilogue per pixel reduces them to RX / ACE.
 //
-// This file holds the preparation kernel and the plain FP32 CUDA-core path
-// (register-blocked 128 x 128 tiles, 8 x 8 outputs per thread, warps skip the
-// all-zero upper-triangle K-chunks of W): the comparator for the tensor-core
-// path in whiten.cu.
+// This file holds the preparation kernel and the plain FP32 CUDA-core path,
+// the comparator for the tensor-core path in rxace_tc.cu and the scorer of
+// frames above its 127 bands.
+//
+// Plain path.  The rows of Waug go in groups of eight; group G multiplies only
+// the bands up to its last row (W is lower triangular; target rows are dense).
+// A persistent block holds all groups' weights in shared memory (118 KB at 224
+// bands and 16 targets) beside the 64 centred pixels of its tile, so the tile's
+// product runs without a barrier, and the next tile's pixels are on their way
+// to registers meanwhile.  A half-warp takes all 64 pixels (four per lane) of
+// one "chain", the groups G, G + 16, G + 32, whose squares form one partial sum
+// of RX.  Chains differ in length, so the host deals them out: neighbours in
+// length share a warp, and each SM sub-partition gets a long and a short warp.
+// Bound: FP32 FMA (B^2 / 2 + T B per pixel).  1024 x 1024 x 224 fp16, 16
+// targets: 3.24 ms with 128 x 128 tiles that staged W and the cube per 16-band
+// chunk for every row tile (16-way conflicts on W's transposing store, a
+// barrier per chunk, warps idling above the diagonal); see the launch below
+// for the time now.
 #include "common.cuh"
 #include "launch_state.h"
+
+#include <algorithm>
 
 namespace hsi_b200 {
 namespace {
 
-constexpr int kRowsTile = 128;  // output rows (bands + targets) per row tile
-constexpr int kPxTile = 128;    // pixels per block tile
-constexpr int kKChunk = 16;
+constexpr int kPxTile = 64;     // pixels per tile
 constexpr int kThreads = 256;
+constexpr int kGroupRows = 8;   // output rows (bands + targets) per group
+constexpr int kChains = 16;     // partial sums of RX per pixel, a half-warp each
+constexpr int kMaxGroups = (HSI_MAX_BANDS + HSI_MAX_FILTERS_PER_PASS) / kGroupRows;
 
-// Prepared operands in the workspace (FP32 path):
-//   waug[(B+T) padded to 128*R][Bk]   row-major, Bk = B rounded up to 16
-//   mean_hi[B], mean_lo[B]            mu = hi + lo (double-float)
-//   uu[T]
+// Where the groups' weights lie (floats from the panels' start, [k][8 rows] of
+// `bands[g]` bands) and which half-warp takes which chain.
+struct Panels {
+  int groups;
+  int kpad;                       // bands rounded up to 8
+  int floats;                     // of all panels
+  int offset[kMaxGroups];
+  short bands[kMaxGroups];
+  unsigned char chain[kChains];   // chain of half-warp h
+};
+
+// Prepared operands in the workspace (FP32 path).
 struct SimtOperands {
-  float* waug;
-  float* mean_hi;
+  float* panels;   // 16-byte aligned
+  float* mean_hi;  // mu = hi + lo (double-float)
   float* mean_lo;
-  float* uu;
-  int rows;   // padded row count (multiple of 128)
-  int kpad;   // padded K (multiple of 16)
+  float* uu;       // [T]
 };
 
 __host__ __device__ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
-// One block per output row of Waug: rows < B copy W, rows B+t compute
-// v_t = W^T u_t in FP64; the rest are zero.
+Panels make_panels(int B, int T) {
+  Panels p{};
+  p.groups = (B + T + kGroupRows - 1) / kGroupRows;
+  p.kpad = round_up(B, kGroupRows);
+  int cost[kChains] = {}, order[kChains];
+  for (int g = 0; g < p.groups; ++g) {
+    // rows above B end their dot product at the diagonal; target rows are dense
+    p.bands[g] = static_cast<short>(std::min((g + 1) * kGroupRows, p.kpad));
+    cost[g % kChains] += p.bands[g];
+  }
+  for (int c = 0; c < kChains; ++c) order[c] = c;
+  std::stable_sort(order, order + kChains, [&](int a, int b) { return cost[a] > cost[b]; });
+  // pairs of neighbours, longest first: pair i on warp i of the first four,
+  // then the remaining pairs shortest first, so that warps w and w + 4 (one
+  // sub-partition) add up alike
+  for (int i = 0; i < kChains / 2; ++i) {
+    const int w = i < 4 ? i : 4 + (7 - i);
+    p.chain[2 * w] = static_cast<unsigned char>(order[2 * i]);
+    p.chain[2 * w + 1] = static_cast<unsigned char>(order[2 * i + 1]);
+  }
+  // the two halves of a warp read their weights at the same band: the second
+  // halves' panels start 64 bytes off, on other banks
+  for (int half = 0; half < 2; ++half) {
+    if (half) p.floats += 16;
+    for (int w = 0; w < kChains / 2; ++w)
+      for (int g = p.chain[2 * w + half]; g < p.groups; g += kChains) {
+        p.offset[g] = p.floats;
+        p.floats += p.bands[g] * kGroupRows;
+      }
+  }
+  return p;
+}
+
+// One thread per weight: rows < B copy W, rows B + t hold v_t = W^T u_t in
+// FP64; the rest are zero.  blockIdx.x: the group, blockIdx.y: 256 weights of
+// its panel.
 __global__ void __launch_bounds__(256) prep_simt_kernel(const double* __restrict__ stats, int B, int T,
-                                                       SimtOperands op) {
-  const int n = blockIdx.x;
+                                                       const __grid_constant__ Panels pn, SimtOperands op) {
+  const int g = blockIdx.x;
   const double* mean = stats;
   const double* W = stats + B;
   const double* tw = W + static_cast<size_t>(B) * B;
   const double* tn = tw + static_cast<size_t>(T) * B;
-  float* row = op.waug + static_cast<size_t>(n) * op.kpad;
-  for (int k = threadIdx.x; k < op.kpad; k += blockDim.x) {
+  const int e = blockIdx.y * 256 + threadIdx.x;
+  if (e < pn.bands[g] * kGroupRows) {
+    const int k = e / kGroupRows, n = g * kGroupRows + e % kGroupRows;
     double v = 0.0;
     if (k < B) {
       if (n < B) {
         v = W[static_cast<size_t>(n) * B + k];
       } else if (n < B + T) {
         const double* u = tw + static_cast<size_t>(n - B) * B;
+#pragma unroll 16
         for (int i = k; i < B; ++i) v += W[static_cast<size_t>(i) * B + k] * u[i];
       }
     }
-    row[k] = static_cast<float>(v);
+    op.panels[pn.offset[g] + e] = static_cast<float>(v);
   }
-  if (n == 0) {
+  if (g == 0 && blockIdx.y == 0) {
     for (int b = threadIdx.x; b < B; b += blockDim.x) {
       const float hi = static_cast<float>(mean[b]);
       op.mean_hi[b] = hi;
@@ -94,180 +153,228 @@ struct ScoreOut {
   int64_t map_stride;
 };
 
-// Epilogue shared by both paths: RX and ACE for one pixel from its z-norm and
-// ACE numerators.  Follows src/detectors_cpu.cpp:127-156.
-__device__ __forceinline__ void write_pixel(const ScoreOut& o, int64_t p, float rx, const float* zu,
-                                            const float* uu, int T) {
-  if (o.rx) o.rx[p] = rx;
-  float best = -1.0f;
-  int32_t best_t = -1;
-  for (int t = 0; t < T; ++t) {
-    float a = 0.0f;
-    if (uu[t] > 0.0f && rx > 0.0f) {
-      a = (zu[t] * zu[t]) / (uu[t] * rx);
-      if (a > best) {
-        best = a;
-        best_t = t;
-      }
-    }
-    if (o.ace_maps) o.ace_maps[static_cast<int64_t>(t) * o.map_stride + p] = a;
-  }
-  if (o.ace_best) o.ace_best[p] = best < 0.0f ? 0.0f : fminf(best, 1.0f);
-  if (o.ace_target) o.ace_target[p] = best_t;
-}
+// V pixels of band row b from pixel p on, centred; zero past the frame.
+template <typename T>
+constexpr int kVec = 16 / static_cast<int>(sizeof(T));
 
 struct SimtSmem {
-  float w[2][kKChunk][kRowsTile];  // W chunk, k-major
-  float y[2][kKChunk][kPxTile];    // Y chunk
-  float rx[16][kPxTile];
-  float zu[HSI_MAX_FILTERS_PER_PASS][kPxTile];
+  float mean_hi[HSI_MAX_BANDS], mean_lo[HSI_MAX_BANDS];
   float uu[HSI_MAX_FILTERS_PER_PASS];
+  float rx[kChains][kPxTile];
+  float zu[HSI_MAX_FILTERS_PER_PASS][kPxTile];
+  // then y[kpad][kPxTile], the panels
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 2) rxace_simt_kernel(const T* __restrict__ cube, int64_t pixels,
-                                                             int64_t stride, int B, int Tn, SimtOperands op,
-                                                             ScoreOut out) {
+// BANDS: the instance's largest padded band count, which sizes the register
+// prefetch.  `aligned`: the cube starts on 16 bytes.
+template <typename T, int BANDS>
+__global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
+    rxace_simt_kernel(const T* __restrict__ cube, int64_t pixels, int64_t stride, int B, int Tn, int aligned,
+                      const __grid_constant__ Panels pn, SimtOperands op, ScoreOut out) {
+  constexpr int V = kVec<T>;
+  constexpr int kRowVecs = kPxTile / V;                                    // 16-byte groups per band row
+  constexpr int kLoads = (BANDS * kRowVecs + kThreads - 1) / kThreads;     // per thread and tile
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SimtSmem& sm = *reinterpret_cast<SimtSmem*>(smem_raw);
-  const int tx = threadIdx.x & 15;  // pixel group: pixels tx*4 .. +3 and 64 + tx*4 .. +3
-  const int ty = threadIdx.x >> 4;  // row group: rows ty*8 .. ty*8 + 7
-  const int64_t p0 = static_cast<int64_t>(blockIdx.x) * kPxTile;
-  const int kchunks = op.kpad / kKChunk;
-  if (threadIdx.x < Tn) sm.uu[threadIdx.x] = op.uu[threadIdx.x];
+  float* ys = reinterpret_cast<float*>(smem_raw + sizeof(SimtSmem));  // [kpad][kPxTile]
+  float* ws = ys + pn.kpad * kPxTile;                                 // panels
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int64_t tiles = div_up<int64_t>(pixels, kPxTile);
 
-  float rx_part[8];
-#pragma unroll
-  for (int j = 0; j < 8; ++j) rx_part[j] = 0.0f;
+  for (int i = tid; i < pn.floats / 4; i += kThreads)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(ws + 4 * i)), "l"(op.panels + 4 * i)
+                 : "memory");
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  for (int b = tid; b < B; b += kThreads) {
+    sm.mean_hi[b] = op.mean_hi[b];
+    sm.mean_lo[b] = op.mean_lo[b];
+  }
+  if (tid < Tn) sm.uu[tid] = op.uu[tid];
 
-  for (int rt = 0; rt < op.rows / kRowsTile; ++rt) {
-    const int r0 = rt * kRowsTile;
-    float2 acc[8][4];  // row i, pixels (2 j2, 2 j2 + 1) of this thread's 8: packed FMAs
+  // this thread's share of a tile: group m of row (tid + 256 m) / kRowVecs
+  uint4 raw[kLoads];
+  auto fetch = [&](int64_t tile) {
+    const int64_t p0 = tile * kPxTile;
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int m = 0; m < kLoads; ++m) {
+      const int e = tid + kThreads * m, b = e / kRowVecs;
+      const int64_t p = p0 + e % kRowVecs * V;
+      raw[m] = make_uint4(0u, 0u, 0u, 0u);
+      if (b >= B || p >= pixels) continue;
+      const T* src = cube + static_cast<int64_t>(b) * stride + p;
+      if (aligned && p + V <= pixels) {
+        raw[m] = __ldg(reinterpret_cast<const uint4*>(src));
+      } else {
+        T v[V];
 #pragma unroll
-      for (int j2 = 0; j2 < 4; ++j2) acc[i][j2] = make_float2(0.0f, 0.0f);
-    // A warp owns rows r0 + 16w .. r0 + 16w + 15; W is zero above the
-    // diagonal, so K-chunks past its last row contribute nothing unless the
-    // warp also holds target rows (dense).
-    const int warp_rows_hi = r0 + (threadIdx.x >> 5) * 16 + 15;
-    const bool warp_dense = warp_rows_hi >= B;
-
-    // The cube elements of chunk kc + 1 are loaded into registers before chunk
-    // kc's FMAs and stored to the other buffer after them, so their latency
-    // overlaps the math.  W (a few hundred KB, resident in L2) is copied then.
-    constexpr int kPer = kKChunk * kPxTile / kThreads;  // 8 cube elements per thread
-    float yreg[kPer];
-    auto fetch = [&](int kc) {
-      const int k0 = kc * kKChunk;
-#pragma unroll
-      for (int m = 0; m < kPer; ++m) {
-        const int e = threadIdx.x + kThreads * m;
-        const int b = k0 + e / kPxTile;
-        const int64_t p = p0 + e % kPxTile;
-        float y = 0.0f;
-        if (b < B && p < pixels)
-          y = (to_f<T>(cube[static_cast<int64_t>(b) * stride + p]) - op.mean_hi[b]) - op.mean_lo[b];
-        yreg[m] = y;
+        for (int j = 0; j < V; ++j) v[j] = p + j < pixels ? src[j] : T(0.0f);
+        raw[m] = *reinterpret_cast<const uint4*>(v);
       }
-    };
-    auto commit = [&](int kc, int buf) {
-      const int k0 = kc * kKChunk;
-      for (int e = threadIdx.x; e < kKChunk * kRowsTile; e += kThreads)
-        sm.w[buf][e % kKChunk][e / kKChunk] = op.waug[static_cast<size_t>(r0 + e / kKChunk) * op.kpad + k0 + e % kKChunk];
+    }
+  };
+  auto commit = [&](int64_t tile) {
+    const int64_t p0 = tile * kPxTile;
 #pragma unroll
-      for (int m = 0; m < kPer; ++m) {
-        const int e = threadIdx.x + kThreads * m;
-        sm.y[buf][e / kPxTile][e % kPxTile] = yreg[m];
-      }
-    };
-    fetch(0);
-    commit(0, 0);
-    __syncthreads();
-    for (int kc = 0; kc < kchunks; ++kc) {
-      const int buf = kc & 1;
-      if (kc + 1 < kchunks) fetch(kc + 1);
-      const bool skip = !warp_dense && kc * kKChunk > warp_rows_hi;
-      if (!skip) {
+    for (int m = 0; m < kLoads; ++m) {
+      const int e = tid + kThreads * m, b = e / kRowVecs, px = e % kRowVecs * V;
+      if (b >= pn.kpad) continue;
+      T v[V];
+      *reinterpret_cast<uint4*>(v) = raw[m];
+      const float hi = b < B ? sm.mean_hi[b] : 0.0f, lo = b < B ? sm.mean_lo[b] : 0.0f;
+      float y[V];
 #pragma unroll
-        for (int k = 0; k < kKChunk; ++k) {
-          const float4 wa = *reinterpret_cast<const float4*>(&sm.w[buf][k][ty * 8]);
-          const float4 wb = *reinterpret_cast<const float4*>(&sm.w[buf][k][ty * 8 + 4]);
-          const float4 ya = *reinterpret_cast<const float4*>(&sm.y[buf][k][tx * 4]);
-          const float4 yb = *reinterpret_cast<const float4*>(&sm.y[buf][k][64 + tx * 4]);
+      for (int j = 0; j < V; ++j) y[j] = b < B && p0 + px + j < pixels ? (to_f<T>(v[j]) - hi) - lo : 0.0f;
+#pragma unroll
+      for (int j = 0; j < V; j += 4)
+        *reinterpret_cast<float4*>(ys + b * kPxTile + px + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+    }
+  };
+
+  int64_t tile = blockIdx.x;
+  fetch(tile);
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  commit(tile);
+  __syncthreads();
+  const int px = 4 * (lane & 15);
+  const int chain = pn.chain[2 * (tid >> 5) + (lane >> 4)];
+  for (; tile < tiles; tile += gridDim.x) {
+    const int64_t next = tile + gridDim.x;
+    if (next < tiles) fetch(next);
+    float rx_part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    for (int g = chain; g < pn.groups; g += kChains) {
+      float2 acc[kGroupRows][2];  // row i, pixel pairs of this lane's four: packed FMAs
+#pragma unroll
+      for (int i = 0; i < kGroupRows; ++i) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
+      const float* w = ws + pn.offset[g];
+      const float* y = ys + px;
+      const int bands = pn.bands[g];  // a multiple of 8
+#pragma unroll 1
+      for (int k0 = 0; k0 < bands; k0 += 8, w += 8 * kGroupRows, y += 8 * kPxTile) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float4 wa = *reinterpret_cast<const float4*>(w + k * kGroupRows);
+          const float4 wb = *reinterpret_cast<const float4*>(w + k * kGroupRows + 4);
+          const float4 yk = *reinterpret_cast<const float4*>(y + k * kPxTile);
           const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-          const float2 yv[4] = {make_float2(ya.x, ya.y), make_float2(ya.z, ya.w), make_float2(yb.x, yb.y),
-                                make_float2(yb.z, yb.w)};
+          const float2 y0 = make_float2(yk.x, yk.y), y1 = make_float2(yk.z, yk.w);
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
+          for (int i = 0; i < kGroupRows; ++i) {
             const float2 wi = make_float2(wv[i], wv[i]);
-#pragma unroll
-            for (int j2 = 0; j2 < 4; ++j2) acc[i][j2] = ffma2(wi, yv[j2], acc[i][j2]);
+            acc[i][0] = ffma2(wi, y0, acc[i][0]);
+            acc[i][1] = ffma2(wi, y1, acc[i][1]);
           }
         }
       }
-      // buffer buf ^ 1 was last read in iteration kc - 1, before its closing barrier
-      if (kc + 1 < kchunks) commit(kc + 1, buf ^ 1);
-      __syncthreads();
-    }
-    // fold: rows < B -> RX partials; rows B..B+T-1 -> ACE numerators
+      // fold: rows < B -> RX partials; rows B..B+T-1 -> ACE numerators
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int row = r0 + ty * 8 + i;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int px = j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4;
-        const float z = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
+      for (int i = 0; i < kGroupRows; ++i) {
+        const int row = g * kGroupRows + i;
+        const float z[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
         if (row < B) {
-          rx_part[j] = fmaf(z, z, rx_part[j]);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) rx_part[j] = fmaf(z[j], z[j], rx_part[j]);
         } else if (row < B + Tn) {
-          sm.zu[row - B][px] = z;
+          *reinterpret_cast<float4*>(&sm.zu[row - B][px]) = make_float4(z[0], z[1], z[2], z[3]);
         }
       }
     }
-  }
-#pragma unroll
-  for (int j = 0; j < 8; ++j) sm.rx[ty][j < 4 ? tx * 4 + j : 64 + tx * 4 + j - 4] = rx_part[j];
-  __syncthreads();
-  if (threadIdx.x < kPxTile) {
-    const int px = threadIdx.x;
-    const int64_t p = p0 + px;
-    if (p < pixels) {
+    *reinterpret_cast<float4*>(&sm.rx[chain][px]) = make_float4(rx_part[0], rx_part[1], rx_part[2], rx_part[3]);
+    __syncthreads();  // the tile's sums are in, its pixels done with
+    if (next < tiles) commit(next);
+    // RX and ACE of one pixel by four lanes, a quarter of the targets each
+    // (reference src/detectors_cpu.cpp:127-156)
+    {
+      const int q = tid & 3, epx = tid >> 2;
+      const int64_t p = tile * kPxTile + epx;
       float rx = 0.0f;
 #pragma unroll
-      for (int g = 0; g < 16; ++g) rx += sm.rx[g][px];
-      float zu[HSI_MAX_FILTERS_PER_PASS];
-      for (int t = 0; t < Tn; ++t) zu[t] = sm.zu[t][px];
-      write_pixel(out, p, rx, zu, sm.uu, Tn);
+      for (int c = 0; c < kChains; ++c) rx += sm.rx[c][epx];
+      float best = -1.0f;
+      int32_t best_t = -1;
+      const int t0 = q * Tn / 4, t1 = (q + 1) * Tn / 4;
+      for (int t = t0; t < t1; ++t) {
+        float a = 0.0f;
+        if (sm.uu[t] > 0.0f && rx > 0.0f) {
+          const float zu = sm.zu[t][epx];
+          a = (zu * zu) / (sm.uu[t] * rx);
+          if (a > best) {
+            best = a;
+            best_t = t;
+          }
+        }
+        if (out.ace_maps && p < pixels) out.ace_maps[static_cast<int64_t>(t) * out.map_stride + p] = a;
+      }
+      // lowest target on ties: a later quarter wins only when strictly larger
+#pragma unroll
+      for (int o = 1; o < 4; o <<= 1) {
+        const float ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int32_t ot = __shfl_xor_sync(0xffffffffu, best_t, o);
+        const bool other_first = (q & o) != 0;
+        if (ob > best || (other_first && ob == best && ot >= 0)) {
+          best = ob;
+          best_t = ot;
+        }
+      }
+      if (q == 0 && p < pixels) {
+        if (out.rx) out.rx[p] = rx;
+        if (out.ace_best) out.ace_best[p] = best < 0.0f ? 0.0f : fminf(best, 1.0f);
+        if (out.ace_target) out.ace_target[p] = best_t;
+      }
     }
+    __syncthreads();  // the next tile's pixels are in, this one's sums read
   }
 }
 
 size_t align256(size_t v) { return (v + 255) & ~static_cast<size_t>(255); }
 
-SimtOperands carve_simt(void* ws, int B, int T) {
+// The size callers have always been asked for (row tiles of 128, bands rounded
+// up to 16); the panels take less than half of it.
+size_t simt_bytes(int B, int T) {
+  return align256(sizeof(float) * static_cast<size_t>(round_up(B + T, 128)) * round_up(B, 16)) +
+         3 * align256(sizeof(float) * HSI_MAX_BANDS);
+}
+
+SimtOperands carve_simt(void* ws, const Panels& pn) {
   SimtOperands op;
-  op.rows = round_up(B + T, kRowsTile);
-  op.kpad = round_up(B, kKChunk);
-  unsigned char* p = static_cast<unsigned char*>(ws);
-  op.waug = reinterpret_cast<float*>(p);
-  p += align256(sizeof(float) * static_cast<size_t>(op.rows) * op.kpad);
-  op.mean_hi = reinterpret_cast<float*>(p);
-  p += align256(sizeof(float) * HSI_MAX_BANDS);
-  op.mean_lo = reinterpret_cast<float*>(p);
-  p += align256(sizeof(float) * HSI_MAX_BANDS);
-  op.uu = reinterpret_cast<float*>(p);
+  const uintptr_t base = (reinterpret_cast<uintptr_t>(ws) + 15u) & ~static_cast<uintptr_t>(15u);
+  op.panels = reinterpret_cast<float*>(base);
+  op.mean_hi = op.panels + round_up(pn.floats, 4);
+  op.mean_lo = op.mean_hi + HSI_MAX_BANDS;
+  op.uu = op.mean_lo + HSI_MAX_BANDS;
   return op;
 }
 
-size_t simt_bytes(int B, int T) {
-  return align256(sizeof(float) * static_cast<size_t>(round_up(B + T, kRowsTile)) * round_up(B, kKChunk)) +
-         3 * align256(sizeof(float) * HSI_MAX_BANDS);
+template <typename T, int BANDS>
+cudaError_t launch_simt(const void* cube, int64_t P, int64_t stride, int B, int Tn, const Panels& pn,
+                        const SimtOperands& op, const ScoreOut& o, cudaStream_t s) {
+  // in steps of 8 KB, so that few layouts are ever asked about
+  const size_t need = sizeof(SimtSmem) + sizeof(float) * (static_cast<size_t>(pn.kpad) * kPxTile + pn.floats);
+  const size_t smem = std::min<size_t>((need + 8191) / 8192 * 8192, 232448);
+  const int resident = device_residency(rxace_simt_kernel<T, BANDS>, kThreads, smem);
+  if (resident <= 0) {
+    const cudaError_t e = raise_smem_limit(rxace_simt_kernel<T, BANDS>, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
+  }
+  const int64_t tiles = div_up<int64_t>(P, kPxTile);
+  const int64_t wave = static_cast<int64_t>(std::max(resident, 1)) * device_sm_count();
+  const int aligned = (reinterpret_cast<uintptr_t>(cube) & 15u) == 0;
+  rxace_simt_kernel<T, BANDS><<<static_cast<unsigned>(std::min(tiles, wave)), kThreads, smem, s>>>(
+      static_cast<const T*>(cube), P, stride, B, Tn, aligned, pn, op, o);
+  return cudaGetLastError();
+}
+
+template <typename T>
+cudaError_t launch_simt_bands(const void* cube, int64_t P, int64_t stride, int B, int Tn, const Panels& pn,
+                              const SimtOperands& op, const ScoreOut& o, cudaStream_t s) {
+  if (pn.kpad <= 64) return launch_simt<T, 64>(cube, P, stride, B, Tn, pn, op, o, s);
+  if (pn.kpad <= 128) return launch_simt<T, 128>(cube, P, stride, B, Tn, pn, op, o, s);
+  return launch_simt<T, 256>(cube, P, stride, B, Tn, pn, op, o, s);
 }
 
 }  // namespace
 
-// Shared with whiten.cu.
+// Shared with rxace_tc.cu.
 int rxace_check(const void* cube, int height, int width, int bands, int dtype, int64_t stride, const double* stats,
                 int T) {
   if (!cube || !stats || height <= 0 || width <= 0 || bands <= 0 || bands > HSI_MAX_BANDS) return HSI_E_INVALID;
@@ -298,21 +405,13 @@ extern "C" HSI_API int hsi_rx_ace_simt(const void* d_cube, int height, int width
   if (d_ace_maps && map_stride < P) return HSI_E_INVALID;
   if (!d_workspace || workspace_bytes < simt_bytes(bands, num_targets)) return HSI_E_WORKSPACE;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  const SimtOperands op = carve_simt(d_workspace, bands, num_targets);
-  prep_simt_kernel<<<op.rows, 256, 0, s>>>(d_stats64, bands, num_targets, op);
+  const Panels pn = make_panels(bands, num_targets);
+  const SimtOperands op = carve_simt(d_workspace, pn);
+  prep_simt_kernel<<<dim3(pn.groups, (pn.kpad * kGroupRows + 255) / 256), 256, 0, s>>>(d_stats64, bands, num_targets,
+                                                                                     pn, op);
   ScoreOut o{d_rx, d_ace_best, d_ace_target, d_ace_maps, map_stride};
-  const unsigned blocks = static_cast<unsigned>(div_up<int64_t>(P, kPxTile));
-  const int smem = static_cast<int>(sizeof(SimtSmem));
-  if (dtype == HSI_F32) {
-    const cudaError_t e = raise_smem_limit(rxace_simt_kernel<float>, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    rxace_simt_kernel<float><<<blocks, kThreads, smem, s>>>(static_cast<const float*>(d_cube), P, plane_stride,
-                                                            bands, num_targets, op, o);
-  } else {
-    const cudaError_t e = raise_smem_limit(rxace_simt_kernel<__half>, smem);
-    if (e != cudaSuccess) return static_cast<int>(e);
-    rxace_simt_kernel<__half><<<blocks, kThreads, smem, s>>>(static_cast<const __half*>(d_cube), P, plane_stride,
-                                                             bands, num_targets, op, o);
-  }
-  return static_cast<int>(cudaGetLastError());
+  const cudaError_t e =
+      dtype == HSI_F32 ? launch_simt_bands<float>(d_cube, P, plane_stride, bands, num_targets, pn, op, o, s)
+                       : launch_simt_bands<__half>(d_cube, P, plane_stride, bands, num_targets, pn, op, o, s);
+  return static_cast<int>(e);
 }

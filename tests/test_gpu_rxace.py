@@ -73,6 +73,45 @@ def test_rx_ace_with_fp64_statistics(hsi, orc, simt, B, T):
     _check_scores(orc, host, S, rx.cpu().numpy(), ace.cpu().numpy(), at.cpu().numpy(), maps.cpu().numpy(), T)
 
 
+@pytest.mark.parametrize("B,T", [(1, 0), (7, 1), (8, 5), (9, 16), (64, 3), (65, 16), (121, 7), (128, 2), (129, 16),
+                                 (200, 1), (249, 15), (256, 16), (256, 0)])
+@pytest.mark.parametrize("dtype,H,W,off", [(0, 5, 13, 0), (1, 9, 71, 0), (0, 131, 149, 1), (1, 8, 8, 3)])
+def test_plain_path_group_and_tile_edges(hsi, orc, B, T, dtype, H, W, off):
+    """Rows that do and do not fill their groups of eight, targets that share a
+    group with bands, one to three groups per partial sum, tiles with a tail,
+    several tiles per block, and cubes `off` elements into an allocation (not on
+    16 bytes).  Only the frame's own elements are readable."""
+    P = H * W
+    rng = np.random.default_rng(1000 * B + 10 * T + H)
+    mix = rng.standard_normal((B, min(B, 6)))
+    many = 4 * B + 200
+    back = (mix @ rng.standard_normal((mix.shape[1], many + P)) * 0.1 + 0.5
+            + 0.02 * rng.standard_normal((B, many + P))).astype(np.float32)
+    lib = (0.5 + 0.1 * rng.standard_normal((T, B))).astype(np.float32)
+    S = _fp64_stats(orc, np.ascontiguousarray(back[:, :many]), lib, 1e-5)
+    stats = torch.from_numpy(_pack(S)).cuda()
+    tdt = torch.float32 if dtype == 0 else torch.float16
+    stride = (P + 7) // 8 * 8
+    store = torch.full((off + (B - 1) * stride + P,), float("nan"), dtype=tdt, device="cuda")
+    scored = torch.from_numpy(back[:, many:].copy()).cuda().to(tdt)
+    for b in range(B):
+        store[off + b * stride:off + b * stride + P] = scored[b]
+    rx = torch.full((P,), np.nan, device="cuda")
+    ace = torch.full((P,), np.nan, device="cuda")
+    at = torch.full((P,), -9, dtype=torch.int32, device="cuda")
+    maps = torch.full((max(T, 1), P), np.nan, device="cuda")
+    hsi.rx_ace(store[off:], H, W, B, stats, T, dtype=dtype, stride=stride, rx=rx, ace_best=ace, ace_target=at,
+               ace_maps=maps, simt=True)
+    torch.cuda.synchronize()
+    host = scored.float().cpu().numpy()
+    if T == 0:
+        rx0 = orc.rx(host, S)
+        assert np.max(np.abs(rx.cpu().numpy() - rx0) / np.maximum(1.0, np.abs(rx0))) <= TOL
+        assert (at == -1).all() and (ace == 0).all()
+        return
+    _check_scores(orc, host, S, rx.cpu().numpy(), ace.cpu().numpy(), at.cpu().numpy(), maps.cpu().numpy(), T)
+
+
 @pytest.mark.parametrize("dtype", [0, 1])
 def test_rx_ace_tensor_core_at_size(hsi, orc, dtype):
     """512 x 512 x 113 with anomalies, 8 targets, both cube types: the tensor-core

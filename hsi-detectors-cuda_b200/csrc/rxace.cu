@@ -21,16 +21,21 @@
 // the bands up to its last row (W is lower triangular; target rows are dense).
 // A persistent block holds all groups' weights in shared memory (118 KB at 224
 // bands and 16 targets) beside the 64 centred pixels of its tile, so the tile's
-// product runs without a barrier, and the next tile's pixels are on their way
-// to registers meanwhile.  A half-warp takes all 64 pixels (four per lane) of
-// one "chain", the groups G, G + 16, G + 32, whose squares form one partial sum
-// of RX.  Chains differ in length, so the host deals them out: neighbours in
-// length share a warp, and each SM sub-partition gets a long and a short warp.
-// Bound: FP32 FMA (B^2 / 2 + T B per pixel).  1024 x 1024 x 224 fp16, 16
-// targets: 3.24 ms with 128 x 128 tiles that staged W and the cube per 16-band
-// chunk for every row tile (16-way conflicts on W's transposing store, a
-// barrier per chunk, warps idling above the diagonal); see the launch below
-// for the time now.
+// product runs without a block barrier, and the next tile's pixels are on their
+// way to registers meanwhile.  A half-warp takes all 64 pixels (four per lane)
+// of one group, a warp a pair of neighbours; the host deals the pairs out so
+// that every warp has the same number of bands to go through (240 each at 224
+// bands and 16 targets: with two warps per sub-partition, one that ends early
+// leaves the other's latencies bare).  The squares of groups G, G + 16, G + 32
+// form one partial sum of RX; a pair waits for the pair eight before it, which
+// is always started earlier, before it adds its own.
+// Bound: FP32 FMA (B^2 / 2 + T B per pixel; the pipe is 71 % busy) and the
+// shared-memory reads beside it (74 %: eight weights and four pixels per lane
+// for 16 packed FMAs; sixteen rows by two pixels needed ten wavefronts where
+// this tile needs eight, and was 13 % slower).  1024 x 1024 x 224 fp16, 16
+// targets: 1.28 ms; 3.24 with 128 x 128 tiles that staged W and the cube per
+// 16-band chunk for every row tile (16-way conflicts on W's transposing store,
+// a barrier per chunk, warps idling above the diagonal).
 #include "common.cuh"
 #include "launch_state.h"
 
@@ -42,18 +47,21 @@ namespace {
 constexpr int kPxTile = 64;     // pixels per tile
 constexpr int kThreads = 256;
 constexpr int kGroupRows = 8;   // output rows (bands + targets) per group
-constexpr int kChains = 16;     // partial sums of RX per pixel, a half-warp each
+constexpr int kChains = 16;     // partial sums of RX per pixel: groups G, G + 16, G + 32 each
 constexpr int kMaxGroups = (HSI_MAX_BANDS + HSI_MAX_FILTERS_PER_PASS) / kGroupRows;
+constexpr int kMaxPairs = (kMaxGroups + 1) / 2;
+constexpr int kWarps = kThreads / 32;
 
 // Where the groups' weights lie (floats from the panels' start, [k][8 rows] of
-// `bands[g]` bands) and which half-warp takes which chain.
+// `bands[g]` bands) and which warp takes which pairs of groups (2 i, 2 i + 1).
 struct Panels {
   int groups;
   int kpad;                       // bands rounded up to 8
   int floats;                     // of all panels
   int offset[kMaxGroups];
   short bands[kMaxGroups];
-  unsigned char chain[kChains];   // chain of half-warp h
+  unsigned char first[kWarps + 1];  // warp w's pairs: pair[first[w]] .. pair[first[w + 1] - 1], ascending
+  unsigned char pair[kMaxPairs];
 };
 
 // Prepared operands in the workspace (FP32 path).
@@ -70,31 +78,31 @@ Panels make_panels(int B, int T) {
   Panels p{};
   p.groups = (B + T + kGroupRows - 1) / kGroupRows;
   p.kpad = round_up(B, kGroupRows);
-  int cost[kChains] = {}, order[kChains];
-  for (int g = 0; g < p.groups; ++g) {
-    // rows above B end their dot product at the diagonal; target rows are dense
+  const int pairs = (p.groups + 1) / 2;
+  for (int g = 0; g < p.groups; ++g)  // rows above B end their dot product at the diagonal; target rows are dense
     p.bands[g] = static_cast<short>(std::min((g + 1) * kGroupRows, p.kpad));
-    cost[g % kChains] += p.bands[g];
+  // longest pair first, each to the warp with the least to do
+  int load[kWarps] = {}, warp_of[kMaxPairs];
+  for (int i = pairs - 1; i >= 0; --i) {
+    const int w = static_cast<int>(std::min_element(load, load + kWarps) - load);
+    warp_of[i] = w;
+    load[w] += p.bands[std::min(2 * i + 1, p.groups - 1)];
   }
-  for (int c = 0; c < kChains; ++c) order[c] = c;
-  std::stable_sort(order, order + kChains, [&](int a, int b) { return cost[a] > cost[b]; });
-  // pairs of neighbours, longest first: pair i on warp i of the first four,
-  // then the remaining pairs shortest first, so that warps w and w + 4 (one
-  // sub-partition) add up alike
-  for (int i = 0; i < kChains / 2; ++i) {
-    const int w = i < 4 ? i : 4 + (7 - i);
-    p.chain[2 * w] = static_cast<unsigned char>(order[2 * i]);
-    p.chain[2 * w + 1] = static_cast<unsigned char>(order[2 * i + 1]);
+  int n = 0;
+  for (int w = 0; w < kWarps; ++w) {
+    p.first[w] = static_cast<unsigned char>(n);
+    for (int i = 0; i < pairs; ++i)
+      if (warp_of[i] == w) p.pair[n++] = static_cast<unsigned char>(i);
   }
-  // the two halves of a warp read their weights at the same band: the second
-  // halves' panels start 64 bytes off, on other banks
+  p.first[kWarps] = static_cast<unsigned char>(n);
+  // the two halves of a warp read their weights at the same band: the odd
+  // groups' panels start 64 bytes off, on other banks
   for (int half = 0; half < 2; ++half) {
     if (half) p.floats += 16;
-    for (int w = 0; w < kChains / 2; ++w)
-      for (int g = p.chain[2 * w + half]; g < p.groups; g += kChains) {
-        p.offset[g] = p.floats;
-        p.floats += p.bands[g] * kGroupRows;
-      }
+    for (int g = half; g < p.groups; g += 2) {
+      p.offset[g] = p.floats;
+      p.floats += p.bands[g] * kGroupRows;
+    }
   }
   return p;
 }
@@ -153,16 +161,17 @@ struct ScoreOut {
   int64_t map_stride;
 };
 
-// V pixels of band row b from pixel p on, centred; zero past the frame.
 template <typename T>
 constexpr int kVec = 16 / static_cast<int>(sizeof(T));
 
 struct SimtSmem {
-  float mean_hi[HSI_MAX_BANDS], mean_lo[HSI_MAX_BANDS];
+  float2 mean[HSI_MAX_BANDS];  // (hi, lo)
   float uu[HSI_MAX_FILTERS_PER_PASS];
   float rx[kChains][kPxTile];
   float zu[HSI_MAX_FILTERS_PER_PASS][kPxTile];
-  // then y[kpad][kPxTile], the panels
+  int done[kMaxPairs + 1];  // tiles whose squares pair i has added (per block, in order)
+  int pad[2];               // y starts on 16 bytes
+  // then y[kpad][kPxTile], the panels, 8 floats that the last band's prefetch reads
 };
 
 // BANDS: the instance's largest padded band count, which sizes the register
@@ -185,50 +194,58 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(ws + 4 * i)), "l"(op.panels + 4 * i)
                  : "memory");
   asm volatile("cp.async.commit_group;" ::: "memory");
-  for (int b = tid; b < B; b += kThreads) {
-    sm.mean_hi[b] = op.mean_hi[b];
-    sm.mean_lo[b] = op.mean_lo[b];
-  }
+  for (int b = tid; b < B; b += kThreads) sm.mean[b] = make_float2(op.mean_hi[b], op.mean_lo[b]);
   if (tid < Tn) sm.uu[tid] = op.uu[tid];
+  if (tid <= kMaxPairs) sm.done[tid] = 0;
 
-  // this thread's share of a tile: group m of row (tid + 256 m) / kRowVecs
+  // this thread's share of a tile: V pixels from px0 on of bands b0, b0 + step, ..
+  constexpr int kStep = kThreads / kRowVecs;
+  const int b0 = tid / kRowVecs, px0 = tid % kRowVecs * V;
+  const T* src0 = cube + static_cast<int64_t>(b0) * stride + px0;
+  const int64_t src_step = kStep * stride;
   uint4 raw[kLoads];
+  const auto whole = [&](int64_t tile) { return aligned && tile * kPxTile + px0 + V <= pixels; };
   auto fetch = [&](int64_t tile) {
-    const int64_t p0 = tile * kPxTile;
+    if (!whole(tile)) return;  // such pixels are read when the tile is stored
+    const T* src = src0 + tile * kPxTile;
 #pragma unroll
-    for (int m = 0; m < kLoads; ++m) {
-      const int e = tid + kThreads * m, b = e / kRowVecs;
-      const int64_t p = p0 + e % kRowVecs * V;
-      raw[m] = make_uint4(0u, 0u, 0u, 0u);
-      if (b >= B || p >= pixels) continue;
-      const T* src = cube + static_cast<int64_t>(b) * stride + p;
-      if (aligned && p + V <= pixels) {
-        raw[m] = __ldg(reinterpret_cast<const uint4*>(src));
-      } else {
+    for (int m = 0; m < kLoads; ++m, src += src_step)
+      if (b0 + m * kStep < B) raw[m] = __ldg(reinterpret_cast<const uint4*>(src));
+  };
+  auto store = [&](int b, const float (&x)[V], int64_t inside) {
+    const float2 mean = sm.mean[b];
+    float y[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) y[j] = j < inside ? (x[j] - mean.x) - mean.y : 0.0f;
+#pragma unroll
+    for (int j = 0; j < V; j += 4)
+      *reinterpret_cast<float4*>(ys + b * kPxTile + px0 + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
+  };
+  auto commit = [&](int64_t tile) {
+    float x[V];
+    if (whole(tile)) {
+#pragma unroll
+      for (int m = 0; m < kLoads; ++m) {
+        if (b0 + m * kStep >= B) break;
         T v[V];
+        *reinterpret_cast<uint4*>(v) = raw[m];
 #pragma unroll
-        for (int j = 0; j < V; ++j) v[j] = p + j < pixels ? src[j] : T(0.0f);
-        raw[m] = *reinterpret_cast<const uint4*>(v);
+        for (int j = 0; j < V; ++j) x[j] = to_f<T>(v[j]);
+        store(b0 + m * kStep, x, V);
+      }
+    } else {
+      const int64_t inside = pixels - (tile * kPxTile + px0);  // may be negative
+      const T* src = src0 + tile * kPxTile;
+#pragma unroll 1
+      for (int b = b0; b < B; b += kStep, src += src_step) {
+#pragma unroll
+        for (int j = 0; j < V; ++j) x[j] = j < inside ? to_f<T>(src[j]) : 0.0f;
+        store(b, x, inside);
       }
     }
   };
-  auto commit = [&](int64_t tile) {
-    const int64_t p0 = tile * kPxTile;
-#pragma unroll
-    for (int m = 0; m < kLoads; ++m) {
-      const int e = tid + kThreads * m, b = e / kRowVecs, px = e % kRowVecs * V;
-      if (b >= pn.kpad) continue;
-      T v[V];
-      *reinterpret_cast<uint4*>(v) = raw[m];
-      const float hi = b < B ? sm.mean_hi[b] : 0.0f, lo = b < B ? sm.mean_lo[b] : 0.0f;
-      float y[V];
-#pragma unroll
-      for (int j = 0; j < V; ++j) y[j] = b < B && p0 + px + j < pixels ? (to_f<T>(v[j]) - hi) - lo : 0.0f;
-#pragma unroll
-      for (int j = 0; j < V; j += 4)
-        *reinterpret_cast<float4*>(ys + b * kPxTile + px + j) = make_float4(y[j], y[j + 1], y[j + 2], y[j + 3]);
-    }
-  };
+  // bands past B multiply zero weights: zero once
+  for (int i = B * kPxTile + tid; i < pn.kpad * kPxTile; i += kThreads) ys[i] = 0.0f;
 
   int64_t tile = blockIdx.x;
   fetch(tile);
@@ -236,50 +253,84 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
   __syncthreads();
   commit(tile);
   __syncthreads();
-  const int px = 4 * (lane & 15);
-  const int chain = pn.chain[2 * (tid >> 5) + (lane >> 4)];
-  for (; tile < tiles; tile += gridDim.x) {
+  const int px = 4 * (lane & 15), half = lane >> 4, warp = tid >> 5;
+  for (int turn = 1; tile < tiles; tile += gridDim.x, ++turn) {
     const int64_t next = tile + gridDim.x;
     if (next < tiles) fetch(next);
-    float rx_part[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-    for (int g = chain; g < pn.groups; g += kChains) {
-      float2 acc[kGroupRows][2];  // row i, pixel pairs of this lane's four: packed FMAs
+    for (int i = pn.first[warp]; i < pn.first[warp + 1]; ++i) {
+      const int pair = pn.pair[i], g = 2 * pair + half;
+      // packed FMAs over row pairs: their weights lie side by side as they are
+      // read, and only the four pixels have to be doubled into a register pair
+      float2 acc[kGroupRows / 2][4];
 #pragma unroll
-      for (int i = 0; i < kGroupRows; ++i) acc[i][0] = acc[i][1] = make_float2(0.0f, 0.0f);
-      const float* w = ws + pn.offset[g];
+      for (int r = 0; r < kGroupRows / 2; ++r)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[r][j] = make_float2(0.0f, 0.0f);
+      const int bands = g < pn.groups ? pn.bands[g] : 0;  // a multiple of 8
+      const float* w = ws + pn.offset[g < pn.groups ? g : 0];
       const float* y = ys + px;
-      const int bands = pn.bands[g];  // a multiple of 8
+      // the next band's operands are read one band ahead
+      float4 wa = *reinterpret_cast<const float4*>(w), wb = *reinterpret_cast<const float4*>(w + 4);
+      float4 yk = *reinterpret_cast<const float4*>(y);
 #pragma unroll 1
-      for (int k0 = 0; k0 < bands; k0 += 8, w += 8 * kGroupRows, y += 8 * kPxTile) {
+      for (int k0 = 0; k0 < bands; k0 += 8) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
-          const float4 wa = *reinterpret_cast<const float4*>(w + k * kGroupRows);
-          const float4 wb = *reinterpret_cast<const float4*>(w + k * kGroupRows + 4);
-          const float4 yk = *reinterpret_cast<const float4*>(y + k * kPxTile);
-          const float wv[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
-          const float2 y0 = make_float2(yk.x, yk.y), y1 = make_float2(yk.z, yk.w);
+          w += kGroupRows;
+          y += kPxTile;
+          const float2 wv[4] = {make_float2(wa.x, wa.y), make_float2(wa.z, wa.w), make_float2(wb.x, wb.y),
+                                make_float2(wb.z, wb.w)};
+          const float yv[4] = {yk.x, yk.y, yk.z, yk.w};
+          wa = *reinterpret_cast<const float4*>(w);
+          wb = *reinterpret_cast<const float4*>(w + 4);
+          yk = *reinterpret_cast<const float4*>(y);
 #pragma unroll
-          for (int i = 0; i < kGroupRows; ++i) {
-            const float2 wi = make_float2(wv[i], wv[i]);
-            acc[i][0] = ffma2(wi, y0, acc[i][0]);
-            acc[i][1] = ffma2(wi, y1, acc[i][1]);
+          for (int j = 0; j < 4; ++j) {
+            const float2 yj = make_float2(yv[j], yv[j]);
+#pragma unroll
+            for (int r = 0; r < kGroupRows / 2; ++r) acc[r][j] = ffma2(wv[r], yj, acc[r][j]);
           }
         }
       }
+      __syncwarp();
       // fold: rows < B -> RX partials; rows B..B+T-1 -> ACE numerators
+      float4 part = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      float* sum = &sm.rx[g % kChains][px];
+      if (pair >= kChains / 2) {
+        // the chain's earlier groups; the wait ends: their warp has them ahead
+        // of anything that waits, and the lowest pair in work waits for none
+        volatile const int* before = &sm.done[pair - kChains / 2];
+        for (uint32_t n = 0; *before < turn && n < kWaitLimit; ++n) {
+        }
+        __threadfence_block();
+        part = *reinterpret_cast<const float4*>(sum);
+      }
+      const auto z_of = [&](int r) {
+        const float2(&a)[4] = acc[r / 2];
+        return r % 2 ? make_float4(a[0].y, a[1].y, a[2].y, a[3].y) : make_float4(a[0].x, a[1].x, a[2].x, a[3].x);
+      };
+      const auto add_square = [&](const float4& z) {
+        part.x = fmaf(z.x, z.x, part.x);
+        part.y = fmaf(z.y, z.y, part.y);
+        part.z = fmaf(z.z, z.z, part.z);
+        part.w = fmaf(z.w, z.w, part.w);
+      };
+      if ((g + 1) * kGroupRows <= B) {
 #pragma unroll
-      for (int i = 0; i < kGroupRows; ++i) {
-        const int row = g * kGroupRows + i;
-        const float z[4] = {acc[i][0].x, acc[i][0].y, acc[i][1].x, acc[i][1].y};
-        if (row < B) {
+        for (int r = 0; r < kGroupRows; ++r) add_square(z_of(r));
+      } else {
 #pragma unroll
-          for (int j = 0; j < 4; ++j) rx_part[j] = fmaf(z[j], z[j], rx_part[j]);
-        } else if (row < B + Tn) {
-          *reinterpret_cast<float4*>(&sm.zu[row - B][px]) = make_float4(z[0], z[1], z[2], z[3]);
+        for (int r = 0; r < kGroupRows; ++r) {
+          const int row = g * kGroupRows + r;
+          if (row < B) add_square(z_of(r));
+          else if (row < B + Tn) *reinterpret_cast<float4*>(&sm.zu[row - B][px]) = z_of(r);
         }
       }
+      *reinterpret_cast<float4*>(sum) = part;
+      __threadfence_block();
+      __syncwarp();
+      if (lane == 0) *const_cast<volatile int*>(&sm.done[pair]) = turn;
     }
-    *reinterpret_cast<float4*>(&sm.rx[chain][px]) = make_float4(rx_part[0], rx_part[1], rx_part[2], rx_part[3]);
     __syncthreads();  // the tile's sums are in, its pixels done with
     if (next < tiles) commit(next);
     // RX and ACE of one pixel by four lanes, a quarter of the targets each
@@ -289,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
       const int64_t p = tile * kPxTile + epx;
       float rx = 0.0f;
 #pragma unroll
-      for (int c = 0; c < kChains; ++c) rx += sm.rx[c][epx];
+      for (int c = 0; c < kChains; ++c) rx += c < pn.groups ? sm.rx[c][epx] : 0.0f;
       float best = -1.0f;
       int32_t best_t = -1;
       const int t0 = q * Tn / 4, t1 = (q + 1) * Tn / 4;
@@ -349,7 +400,7 @@ template <typename T, int BANDS>
 cudaError_t launch_simt(const void* cube, int64_t P, int64_t stride, int B, int Tn, const Panels& pn,
                         const SimtOperands& op, const ScoreOut& o, cudaStream_t s) {
   // in steps of 8 KB, so that few layouts are ever asked about
-  const size_t need = sizeof(SimtSmem) + sizeof(float) * (static_cast<size_t>(pn.kpad) * kPxTile + pn.floats);
+  const size_t need = sizeof(SimtSmem) + sizeof(float) * (static_cast<size_t>(pn.kpad) * kPxTile + pn.floats + kGroupRows);
   const size_t smem = std::min<size_t>((need + 8191) / 8192 * 8192, 232448);
   const int resident = device_residency(rxace_simt_kernel<T, BANDS>, kThreads, smem);
   if (resident <= 0) {

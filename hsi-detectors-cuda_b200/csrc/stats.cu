@@ -142,15 +142,16 @@ __device__ __forceinline__ uint32_t sw128_byte(int row, int k) {
   return static_cast<uint32_t>((row >> 3) * 1024 + (row & 7) * 128 + ((((k >> 4) ^ (row & 7))) << 4) + (k & 15));
 }
 
+// Four consecutive elements as they lie in shared memory, so that the loads of
+// several rows are in flight before any is converted.
 template <typename T>
-__device__ __forceinline__ float4 load4f(const T* p);
-template <>
-__device__ __forceinline__ float4 load4f<float>(const float* p) {
-  return *reinterpret_cast<const float4*>(p);
+using Raw4 = std::conditional_t<sizeof(T) == 4, float4, uint2>;
+template <typename T>
+__device__ __forceinline__ Raw4<T> load_raw4(const T* p) {
+  return *reinterpret_cast<const Raw4<T>*>(p);
 }
-template <>
-__device__ __forceinline__ float4 load4f<__half>(const __half* p) {
-  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+__device__ __forceinline__ float4 to_f4(const float4& v) { return v; }
+__device__ __forceinline__ float4 to_f4(const uint2& raw) {
   const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&raw.x));
   const float2 b = __half22float2(*reinterpret_cast<const __half2*>(&raw.y));
   return make_float4(a.x, a.y, b.x, b.y);
@@ -483,11 +484,14 @@ __global__ void __launch_bounds__(kThreads, 1) stats_gemm_kernel(const __grid_co
       // One half K-block.  `full`: all 64 pixels lie in the frame (every K-block
       // but a frame's last), so no per-pixel validity test is needed.
       auto convert_half = [&](auto full, const T* in, int sub_off, unsigned char* op, int half, int nvalid) {
+        Raw4<T> raw[kSlots];
+#pragma unroll
+        for (int t2 = 0; t2 < kSlots; ++t2) raw[t2] = load_raw4<T>(in + (band0 + 32 * t2) * kBoxPx + sub_off + lp);
 #pragma unroll
         for (int t2 = 0; t2 < kSlots; ++t2) {
           const uint32_t o = (o0 + 4096u * t2) ^ (half ? 64u : 0u);
           if (is_band[t2]) {
-            const float4 x = load4f<T>(in + (band0 + 32 * t2) * kBoxPx + sub_off + lp);
+            const float4 x = to_f4(raw[t2]);
             const float xv[4] = {x.x, x.y, x.z, x.w};
             uint32_t y[4];
 #pragma unroll

@@ -23,6 +23,16 @@
 // shared memory turns from the matrix into L and then into W in place (the
 // target vectors in the caller's workspace), and beyond that the matrices
 // live in the workspace.  The solves use the explicit inverses.
+// What bounds it is latency: one warp's diagonal blocks, the block barriers and
+// the solves.  224 bands and 16 targets, both chains: 310 us (430 with the
+// diagonal's update and inverse as chains of one warp, a lane per row and
+// target in the solves, and 64-bit divisions for every output index); 113
+// bands and 8 targets 60 us.
+// Tried: two diagonal blocks through the register tiles and every product on
+// the FP64 tensor pipe (mma.sync m8n8k4) took 218 us at 224 bands.  Its sums
+// run in another order, so the FP32 weights that the scorers make of them round
+// differently here and there and a best target within a rounding of the next
+// may change: left out.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -81,13 +91,21 @@ __device__ __forceinline__ double warp_sum(double v) {
 __device__ void fill_matrix(double* A, const double* outer, const double* mean, double N, double loading, int n,
                             bool centred) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  constexpr int kIter = HSI_MAX_BANDS / 32;
   for (int i = warp; i < n; i += kWarps) {
     double* ri = A + row_off(i);
-    for (int j = lane; j <= i; j += 32) {
-      double v = outer[static_cast<size_t>(i) * n + j] / N;
-      if (centred) v -= mean[i] * mean[j];
-      if (i == j) v += loading;
-      ri[j] = v;
+    const double* src = outer + static_cast<size_t>(i) * n;
+    double v[kIter];  // a row's loads, then its divisions, in flight together
+#pragma unroll
+    for (int k = 0; k < kIter; ++k) v[k] = lane + 32 * k <= i ? src[lane + 32 * k] : 0.0;
+#pragma unroll
+    for (int k = 0; k < kIter; ++k) {
+      const int j = lane + 32 * k;
+      if (j > i) break;
+      double x = v[k] / N;
+      if (centred) x -= mean[i] * mean[j];
+      if (i == j) x += loading;
+      ri[j] = x;
     }
   }
   __syncthreads();
@@ -118,57 +136,58 @@ constexpr int kHybridMaxBands = 238;  // the largest n with inplace_core(n) doub
 // 1), and W_IJ = -V_II sum_{K=J}^{I-1} L_IK W_KJ for all J < I at once.
 
 // Step 1 (one warp): factor the diagonal block at k0 (kb <= kNb rows) in
-// registers, lane l holding row l.  Writes L_kk into A, V = L_kk^-1 into W's
-// diagonal block and densely into vs[row * kNb + col].  Sets *bad if a pivot
-// is not positive (or NaN).  Not inlined: its 48 doubles of registers would
-// otherwise be allocated across the whole kernel, whose other paths then spill.
+// registers, lane l holding row l, and invert its factor, lane l holding column
+// l of V = L_kk^-1.  Both eliminate with column k as soon as it is known: the
+// shuffles that broadcast it serve both, and no chain is longer than the
+// column's own (the inverse by rows was one chain of 120 FMAs).  Writes L_kk
+// into A, V into W's diagonal block and densely into vs[row * kNb + col].  Sets
+// *bad if a pivot is not positive (or NaN).  Not inlined: its doubles' registers
+// would otherwise be allocated across the whole kernel, whose other paths then
+// spill.
 __device__ __noinline__ void diag_block(double* A, double* W, double* vs, int k0, int kb, int* bad) {
   const int l = threadIdx.x & 31;
   constexpr unsigned kAll = 0xffffffffu;
-  double a[kNb];
+  double a[kNb], v[kNb];
+  double* row = A + ro32(k0 + min(l, kb - 1)) + k0;
 #pragma unroll
-  for (int m = 0; m < kNb; ++m) a[m] = (l < kb && m <= l) ? A[row_off(k0 + l) + k0 + m] : 0.0;
-  double rd[kNb];
+  for (int m = 0; m < kNb; ++m) {
+    a[m] = (l < kb && m <= l) ? row[m] : 0.0;
+    v[m] = m == l ? 1.0 : 0.0;
+  }
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < kNb; ++k) {
-    rd[k] = 0.0;
     if (k < kb) {
       const double akk = __shfl_sync(kAll, a[k], k);
       ok = ok && akk > 0.0;
       const double inv = rsqrt(akk);  // one dependent FP64 op per step instead of a root and a division
       const double sq = akk * inv;
-      rd[k] = inv;
       if (l == k) a[k] = sq;
       else if (l > k) a[k] *= inv;
+      v[k] = k >= l ? v[k] * inv : 0.0;
 #pragma unroll
       for (int j = k + 1; j < kNb; ++j) {
         const double ljk = __shfl_sync(kAll, a[k], j);
         if (l >= j) a[j] -= a[k] * ljk;
+        v[j] -= ljk * v[k];
       }
+    } else {
+      v[k] = 0.0;
     }
   }
-  // V = L^-1, lane l computing column l by forward substitution
-  double v[kNb];
-#pragma unroll
-  for (int i = 0; i < kNb; ++i) {
-    double t = i == l ? 1.0 : 0.0;
-#pragma unroll
-    for (int m = 0; m < i; ++m) t -= __shfl_sync(kAll, a[m], i) * v[m];
-    v[i] = (i >= l && i < kb) ? t * rd[i] : 0.0;
-  }
   if (l < kb) {
-    double* ar = A + row_off(k0 + l) + k0;
 #pragma unroll
     for (int m = 0; m < kNb; ++m)
-      if (m <= l) ar[m] = a[m];
+      if (m <= l) row[m] = a[m];
   }
   __syncwarp();  // L_kk before V over it, when W is A (the in-place path)
   if (l < kNb) {
+    double* w = W + ro32(k0) + k0 + l;  // row k0 + i starts k0 + i + 1 doubles after the row above
 #pragma unroll
     for (int i = 0; i < kNb; ++i) {
       vs[i * kNb + l] = v[i];
-      if (i >= l && i < kb && l < kb) W[row_off(k0 + i) + k0 + l] = v[i];
+      if (i >= l && i < kb && l < kb) *w = v[i];
+      w += k0 + i + 1;
     }
   }
   if (!ok && l == 0) *bad = 1;
@@ -292,31 +311,59 @@ __device__ __forceinline__ bool cholesky_inplace(double* A, int n, double* vs, i
     __syncthreads();
     const int nb2 = min(kNb, rows);  // rows of the next diagonal block
     if (warp == 0) {
-      // the next diagonal block's own update, then its factorisation
-      for (int e = lane; e < nb2 * nb2; e += 32) {
-        const int i = e / nb2, j = e % nb2;
-        if (j > i) continue;
+      // the next diagonal block's own update (a lane takes half a row), then its factorisation
+      const int i = lane >> 1, j0 = 8 * (lane & 1);
+      if (i < nb2) {
         const double* li = A + ro32(r0 + i) + k0;
-        const double* lj = A + ro32(r0 + j) + k0;
-        double t[4] = {0.0, 0.0, 0.0, 0.0};
+        double* ai = A + ro32(r0 + i) + r0;
+        double x[kNb];
 #pragma unroll
-        for (int m = 0; m < kNb; ++m) t[m & 3] += li[m] * lj[m];
-        A[ro32(r0 + i) + r0 + j] -= (t[0] + t[1]) + (t[2] + t[3]);
+        for (int m = 0; m < kNb; ++m) x[m] = li[m];
+#pragma unroll 2
+        for (int j = j0; j < min(j0 + 8, i + 1); ++j) {
+          const double* lj = A + ro32(r0 + j) + k0;
+          double t[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+          for (int m = 0; m < kNb; ++m) t[m & 3] += x[m] * lj[m];
+          ai[j] -= (t[0] + t[1]) + (t[2] + t[3]);
+        }
       }
       __syncwarp();
       diag_block(A, A, vs, r0, nb2, bad);
     } else {
       // the trailing rows past the next block (their columns r0.. only; the
-      // panel columns k0.. that warp 0 reads are not written here)
-      for (int i = nb2 + warp - 1; i < rows; i += kWarps - 1) {
-        const double* li = A + ro32(r0 + i) + k0;
-        double* ai = A + ro32(r0 + i) + r0;
-        for (int j = lane; j <= i; j += 32) {
-          const double* lj = A + ro32(r0 + j) + k0;
-          double t[4] = {0.0, 0.0, 0.0, 0.0};  // four partial sums: a quarter of the dependent chain
+      // panel columns k0.. that warp 0 reads are not written here): four rows
+      // and two columns per lane, one shared-memory read per FMA where a
+      // single result takes three
+      constexpr int kR = 4;
+      for (int i = nb2 + kR * (warp - 1); i < rows; i += kR * (kWarps - 1)) {
+        unsigned li[kR];
 #pragma unroll
-          for (int m = 0; m < kNb; ++m) t[m & 3] += li[m] * lj[m];
-          ai[j] -= (t[0] + t[1]) + (t[2] + t[3]);
+        for (int q = 0; q < kR; ++q) li[q] = ro32(r0 + min(i + q, rows - 1)) + k0;
+        for (int j = lane; j < i + kR; j += 64) {
+          const int j1 = j + 32;
+          const unsigned l0 = ro32(r0 + min(j, rows - 1)) + k0, l1 = ro32(r0 + min(j1, rows - 1)) + k0;
+          double t[kR][2][4];
+#pragma unroll
+          for (int q = 0; q < kR; ++q)
+#pragma unroll
+            for (int m = 0; m < 4; ++m) t[q][0][m] = t[q][1][m] = 0.0;
+#pragma unroll
+          for (int m = 0; m < kNb; ++m) {
+            const double y0 = A[l0 + m], y1 = A[l1 + m];
+#pragma unroll
+            for (int q = 0; q < kR; ++q) {
+              const double x = A[li[q] + m];
+              t[q][0][m & 3] += x * y0;  // four partial sums: a quarter of the dependent chain
+              t[q][1][m & 3] += x * y1;
+            }
+          }
+#pragma unroll
+          for (int q = 0; q < kR; ++q) {
+            double* ai = A + (li[q] - k0 + r0);
+            if (i + q < rows && j <= i + q) ai[j] -= (t[q][0][0] + t[q][0][1]) + (t[q][0][2] + t[q][0][3]);
+            if (i + q < rows && j1 <= i + q) ai[j1] -= (t[q][1][0] + t[q][1][1]) + (t[q][1][2] + t[q][1][3]);
+          }
         }
       }
     }
@@ -642,8 +689,165 @@ __device__ bool chol_inv_tiles(const double* outer, const double* mean, double N
   return true;
 }
 
+// ---- products of W with a chunk of targets -----------------------------------
+//
+// A lane takes a row (column) of W, a warp 32 of them and four targets, up to
+// two such items per warp.  The vectors pass through shared memory `span` bands
+// at a time, [band][kChunk], so that a lane reads its four targets of a band
+// together.  (A lane per row and target reads W once per target, and vectors
+// in the workspace cost a trip to L2 every few bands: 80k cycles per product at
+// 224 bands and 16 targets.)  Each result is four partial sums over every
+// fourth element, counted from its first, (s0 + s1) + (s2 + s3), and up to
+// three left over that join s0.
+
+constexpr int kStageBands = 64;
+
+template <typename V>
+__device__ __forceinline__ void stage_bands(double* stage, int span, int j0, int n, int nt, const V value) {
+  __syncthreads();
+  for (int e = threadIdx.x; e < span * kChunk; e += kThreads) {
+    const int j = j0 + e / kChunk, t = e % kChunk;
+    stage[e] = j < n && t < nt ? value(j, t) : 0.0;
+  }
+  __syncthreads();
+}
+
+struct TargetSums {
+  double s[4][4];  // [target][element mod 4]
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+#pragma unroll
+      for (int p = 0; p < 4; ++p) s[t][p] = 0.0;
+  }
+  template <int P>
+  __device__ __forceinline__ void add(double m, const double* v) {
+    const double2 a = *reinterpret_cast<const double2*>(v), b = *reinterpret_cast<const double2*>(v + 2);
+    s[0][P] += m * a.x;
+    s[1][P] += m * a.y;
+    s[2][P] += m * b.x;
+    s[3][P] += m * b.y;
+  }
+};
+
+// out[t][i] = sum_{j <= i} M[i][j] v(j, t) (M packed lower), t < nt.  span: a
+// multiple of 4.
+template <typename V>
+__device__ __forceinline__ void lower_matvec(const double* M, const V v, double* stage, int span, double* out, int n,
+                                             int nt) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blocks = (n + 31) / 32, groups = (nt + 3) / 4;
+  TargetSums sums[2];
+  sums[0].clear();
+  sums[1].clear();
+  for (int j0 = 0; j0 < n; j0 += span) {
+    stage_bands(stage, span, j0, n, nt, v);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int item = blocks * groups - 1 - warp - q * kWarps;  // the longest rows first
+      if (item < 0) continue;
+      const int i = item / groups * 32 + lane, t0 = item % groups * 4;
+      if (i >= n) continue;
+      const double* mi = M + row_off(i);
+      const double* sv = stage + t0 - j0 * kChunk;
+      const int whole = (i + 1) & ~3, end = min(whole, j0 + span);  // elements in fours
+#pragma unroll 2
+      for (int j = j0; j < end; j += 4) {
+        const double m0 = mi[j], m1 = mi[j + 1], m2 = mi[j + 2], m3 = mi[j + 3];
+        sums[q].add<0>(m0, sv + j * kChunk);
+        sums[q].add<1>(m1, sv + (j + 1) * kChunk);
+        sums[q].add<2>(m2, sv + (j + 2) * kChunk);
+        sums[q].add<3>(m3, sv + (j + 3) * kChunk);
+      }
+      for (int j = max(whole, j0); j <= i && j < j0 + span; ++j) sums[q].add<0>(mi[j], sv + j * kChunk);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int item = blocks * groups - 1 - warp - q * kWarps;
+    const int i = item / groups * 32 + lane, t0 = item % groups * 4;
+    if (item < 0 || i >= n) continue;
+#pragma unroll
+    for (int t = 0; t < 4; ++t)
+      if (t0 + t < nt)
+        out[(t0 + t) * n + i] = (sums[q].s[t][0] + sums[q].s[t][1]) + (sums[q].s[t][2] + sums[q].s[t][3]);
+  }
+  __syncthreads();
+}
+
+// out[t][i] = sum_{k >= i} M[k][i] v(k, t) (M^T, M packed lower), t < nt.  The
+// warp walks the bands together; band k is element k - i of lane i's sum, so
+// that the sums are kept by k mod 4 and told apart by i mod 4 at the end.
+template <typename V>
+__device__ __forceinline__ void upper_matvec(const double* M, const V v, double* stage, int span, double* out, int n,
+                                             int nt) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int blocks = (n + 31) / 32, groups = (nt + 3) / 4;
+  TargetSums sums[2];
+  sums[0].clear();
+  sums[1].clear();
+  for (int k0 = 0; k0 < n; k0 += span) {
+    stage_bands(stage, span, k0, n, nt, v);
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+      const int item = warp + q * kWarps;
+      if (item >= blocks * groups) continue;
+      const int c0 = item / groups * 32, i = c0 + lane, t0 = item % groups * 4;
+      const int tail = n - ((n - min(i, n)) & 3);  // bands from here on join the first sum
+      const double* sv = stage + t0 - k0 * kChunk;
+      const int lo = max(k0, c0), hi = min(n, k0 + span);
+      const double* mk = M + row_off(lo) + i;
+      auto element = [&](int k, int end) {  // zero outside lane i's whole fours
+        double m = 0.0;
+        if (k >= i && k < end) m = *mk;
+        mk += k + 1;
+        return m;
+      };
+#pragma unroll 1
+      for (int k = lo; k < hi; k += 4) {  // lo is a multiple of 4
+        const double m0 = element(k, min(tail, hi)), m1 = element(k + 1, min(tail, hi));
+        const double m2 = element(k + 2, min(tail, hi)), m3 = element(k + 3, min(tail, hi));
+        sums[q].add<0>(m0, sv + k * kChunk);
+        sums[q].add<1>(m1, sv + (k + 1) * kChunk);
+        sums[q].add<2>(m2, sv + (k + 2) * kChunk);
+        sums[q].add<3>(m3, sv + (k + 3) * kChunk);
+      }
+      if (i < n) {
+        for (int k = max(tail, k0); k < hi; ++k) {
+          const double m = M[row_off(k) + i];
+          switch (i & 3) {
+            case 0: sums[q].add<0>(m, sv + k * kChunk); break;
+            case 1: sums[q].add<1>(m, sv + k * kChunk); break;
+            case 2: sums[q].add<2>(m, sv + k * kChunk); break;
+            default: sums[q].add<3>(m, sv + k * kChunk); break;
+          }
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int item = warp + q * kWarps;
+    const int i = item / groups * 32 + lane, t0 = item % groups * 4;
+    if (item >= blocks * groups || i >= n) continue;
+#pragma unroll
+    for (int t = 0; t < 4; ++t) {
+      const double(&s)[4] = sums[q].s[t];
+      // elements 0 and 1 of every four, and 2 and 3, by the first one's place
+      const double e01 = (i & 1) ? s[1] + s[2] : s[0] + s[1], e23 = (i & 1) ? s[3] + s[0] : s[2] + s[3];
+      if (t0 + t < nt) out[(t0 + t) * n + i] = e01 + e23;
+    }
+  }
+  __syncthreads();
+}
+
+// The same sums with a thread per row and target, for one round of them: short
+// code, where the staged products' longer code, run once, costs 2 us of
+// instruction fetches (16 bands and 8 targets: 12.3 us against 14.5; 64 and 8:
+// 26.7 both; 64 and 16, two rounds: 32.8 against 28.7).
+constexpr int kDirectOutputs = kThreads;
 // out[t][i] = sum_{j <= i} M[i][j] v[t][j] (M packed lower), t < nt.
-__device__ void lower_matvec(const double* M, const double* v, double* out, int n, int nt) {
+__device__ void lower_direct(const double* M, const double* v, double* out, int n, int nt) {
   for (int e = threadIdx.x; e < nt * n; e += blockDim.x) {
     const int t = e / n, i = e % n;
     const double* mi = M + row_off(i);
@@ -663,7 +867,7 @@ __device__ void lower_matvec(const double* M, const double* v, double* out, int 
 }
 
 // out[t][i] = sum_{k >= i} M[k][i] v[t][k] (M^T, M packed lower), t < nt.
-__device__ void upper_matvec(const double* M, const double* v, double* out, int n, int nt) {
+__device__ void upper_direct(const double* M, const double* v, double* out, int n, int nt) {
   for (int e = threadIdx.x; e < nt * n; e += blockDim.x) {
     const int t = e / n, i = e % n;
     const double* vt = v + static_cast<size_t>(t) * n;
@@ -679,6 +883,13 @@ __device__ void upper_matvec(const double* M, const double* v, double* out, int 
     out[e] = (s[0] + s[1]) + (s[2] + s[3]);
   }
   __syncthreads();
+}
+
+// Doubles of shared memory ahead of the targets' stage, but for the in-place path.
+__host__ __device__ inline size_t own_doubles(int B) {
+  const size_t vectors =
+      static_cast<size_t>(B) + 2 * static_cast<size_t>(kChunk) * B + lp_elems(B) + kNb * kNb + kTileShared;
+  return vectors + (B <= kTileMaxBands ? tri(B) : B <= kSmemMaxBands ? 2 * tri(B) : 0);
 }
 
 // One cluster of two CTAs per frame, on two SMs at once:
@@ -704,13 +915,14 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   float* cem32 = args.cem32 ? args.cem32 + static_cast<size_t>(f) * T * B : nullptr;
   const bool in_smem = B <= kSmemMaxBands;
   const bool inplace = !in_smem && B <= kHybridMaxBands;
-  // smem: mean[B], two chunk buffers of kChunk x B, the panel / block-row
-  // buffer, the diagonal block's inverse, then the packed matrices (in the
-  // workspace when B is large).  The in-place path keeps only mean, the
-  // diagonal block's inverse and one matrix in shared memory.
+  // smem: mean[B], two products of W with a target chunk (kChunk x B each), the
+  // panel / block-row buffer, the diagonal block's inverse, then the packed
+  // matrices (in the workspace when B is large) and the targets' stage.  The
+  // in-place path keeps only mean, the diagonal block's inverse and one matrix
+  // in shared memory.
   double* mean = smem;
-  double* vec = mean + B;
-  double* buf = vec + static_cast<size_t>(kChunk) * B;
+  double* xs = mean + B;
+  double* buf = xs + static_cast<size_t>(kChunk) * B;
   double* lp = buf + static_cast<size_t>(kChunk) * B;
   double* vs = lp + lp_elems(B);
   double* cbuf = vs + kNb * kNb;  // the tile path's panel, Dinv and flag (kTileShared doubles, 16-byte aligned)
@@ -722,10 +934,20 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   if (inplace) {
     vs = mean + B;
     A = W = vs + kNb * kNb;
-    vec = ws;
-    buf = vec + static_cast<size_t>(kChunk) * B;
+    xs = ws;
+    buf = xs + static_cast<size_t>(kChunk) * B;
     lp = inplace_tb_in_smem(B) ? A + tri(B) : buf + static_cast<size_t>(kChunk) * B;
   }
+  // where the targets pass through: on the in-place path the inverse's block-row
+  // buffer, or the diagonal block's inverse when that buffer is in the workspace
+  int span = kStageBands;
+  size_t stage_at = own_doubles(B);
+  if (inplace) {
+    const bool room = inplace_tb_in_smem(B);
+    stage_at = room ? B + kNb * kNb + tri(B) : B;
+    if (!room) span = 12;  // 192 of kNb * kNb doubles
+  }
+  double* stage = smem + ((stage_at + 1) & ~static_cast<size_t>(1));  // 16-byte rows
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const size_t off_tw = static_cast<size_t>(B) + static_cast<size_t>(B) * B;
   const size_t off_tn = off_tw + static_cast<size_t>(T) * B;
@@ -769,19 +991,30 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
           if (out64) out64[i] = mean[i];
           if (out32) out32[i] = static_cast<float>(mean[i]);
         }
-        for (size_t e = threadIdx.x; e < static_cast<size_t>(B) * B; e += blockDim.x) {
-          const int i = static_cast<int>(e / B), j = static_cast<int>(e % B);
-          const double v = j <= i ? W[row_off(i) + j] : 0.0;
-          if (out64) out64[B + e] = v;
-          if (out32) out32[B + e] = static_cast<float>(v);
+        // a warp per row: an element's row and column by 64-bit division cost more than its stores
+        for (int i = warp; i < B; i += kWarps) {
+          const double* wi = W + row_off(i);
+          const size_t o = B + static_cast<size_t>(i) * B;
+          for (int j = lane; j < B; j += 32) {
+            const double v = j <= i ? wi[j] : 0.0;
+            if (out64) out64[o + j] = v;
+            if (out32) out32[o + j] = static_cast<float>(v);
+          }
         }
         // ACE: u_t = W (d_t - mu) and |u_t|^2, kChunk targets at a time
         for (int t0 = 0; t0 < T; t0 += kChunk) {
           const int nt = min(kChunk, T - t0);
-          for (int e = threadIdx.x; e < nt * B; e += blockDim.x)
-            vec[e] = static_cast<double>(lib[static_cast<size_t>(t0) * B + e]) - mean[e % B];
-          __syncthreads();
-          lower_matvec(W, vec, buf, B, nt);
+          if (nt * B <= kDirectOutputs) {
+            for (int e = threadIdx.x; e < nt * B; e += blockDim.x)
+              xs[e] = static_cast<double>(lib[static_cast<size_t>(t0) * B + e]) - mean[e % B];
+            __syncthreads();
+            lower_direct(W, xs, buf, B, nt);
+          } else {
+            lower_matvec(
+                W,
+                [&](int j, int t) { return static_cast<double>(lib[static_cast<size_t>(t0 + t) * B + j]) - mean[j]; },
+                stage, span, buf, B, nt);
+          }
           for (int e = threadIdx.x; e < nt * B; e += blockDim.x) {
             if (out64) out64[off_tw + static_cast<size_t>(t0) * B + e] = buf[e];
             if (out32) out32[off_tw + static_cast<size_t>(t0) * B + e] = static_cast<float>(buf[e]);
@@ -802,17 +1035,24 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
         // w_t = x_t / |y_t|^2, 0 if that gain is not positive (src/detector.cpp:128-148)
         for (int t0 = 0; t0 < T; t0 += kChunk) {
           const int nt = min(kChunk, T - t0);
-          for (int e = threadIdx.x; e < nt * B; e += blockDim.x)
-            vec[e] = static_cast<double>(lib[static_cast<size_t>(t0) * B + e]);
-          __syncthreads();
-          lower_matvec(W, vec, buf, B, nt);   // y
-          upper_matvec(W, buf, vec, B, nt);   // x (d is no longer needed)
+          if (nt * B <= kDirectOutputs) {
+            for (int e = threadIdx.x; e < nt * B; e += blockDim.x)
+              xs[e] = static_cast<double>(lib[static_cast<size_t>(t0) * B + e]);
+            __syncthreads();
+            lower_direct(W, xs, buf, B, nt);  // y
+            upper_direct(W, buf, xs, B, nt);  // x (d is no longer needed)
+          } else {
+            lower_matvec(
+                W, [&](int j, int t) { return static_cast<double>(lib[static_cast<size_t>(t0 + t) * B + j]); }, stage,
+                span, buf, B, nt);  // y
+            upper_matvec(W, [&](int k, int t) { return buf[t * B + k]; }, stage, span, xs, B, nt);  // x
+          }
           for (int t = warp; t < nt; t += kWarps) {
             double g = 0.0;
             for (int i = lane; i < B; i += 32) g += buf[t * B + i] * buf[t * B + i];
             g = warp_sum(g);
             for (int i = lane; i < B; i += 32) {
-              const double w = g > 0.0 ? vec[t * B + i] / g : 0.0;
+              const double w = g > 0.0 ? xs[t * B + i] / g : 0.0;
               const size_t o = static_cast<size_t>(t0 + t) * B + i;
               if (out64) out64[off_cw + o] = w;
               if (out32) out32[off_cw + o] = static_cast<float>(w);
@@ -832,14 +1072,10 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   if (chain == 0 && threadIdx.x == 0 && args.status) args.status[f] = code != HSI_OK ? code : s_partner_code;
 }
 
-size_t smem_bytes(int B, int /*T*/) {
-  const size_t vectors =
-      static_cast<size_t>(B) + 2 * static_cast<size_t>(kChunk) * B + lp_elems(B) + kNb * kNb + kTileShared;
-  if (B <= kTileMaxBands) return sizeof(double) * (vectors + tri(B));
-  if (B <= kSmemMaxBands) return sizeof(double) * (vectors + 2 * tri(B));
-  if (B <= kHybridMaxBands)
+size_t smem_bytes(int B) {
+  if (B > kSmemMaxBands && B <= kHybridMaxBands)
     return sizeof(double) * (inplace_core(B) + (inplace_tb_in_smem(B) ? kNb * last_block_row(B) : 0));
-  return sizeof(double) * vectors;
+  return sizeof(double) * (own_doubles(B) + 1 + kStageBands * kChunk);
 }
 
 }  // namespace
@@ -884,7 +1120,7 @@ extern "C" HSI_API int hsi_build_statistics(int num_frames, int bands, int num_t
   a.cem32 = d_cem_weights;
   a.status = d_status;
   a.scratch = static_cast<double*>(d_workspace);
-  const size_t smem = smem_bytes(bands, num_targets);
+  const size_t smem = smem_bytes(bands);
   if (smem > 227 * 1024) return HSI_E_CAPACITY;
   const cudaError_t e = raise_smem_limit(factor_kernel, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);

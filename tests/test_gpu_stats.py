@@ -128,6 +128,45 @@ def test_factor_matches_fp64_oracle(hsi, orc, B, T):
     np.testing.assert_array_equal(g32["whitener"], got["whitener"].astype(np.float32))
 
 
+@pytest.mark.parametrize("B,T", [(1, 1), (4, 3), (31, 5), (124, 17), (125, 16), (128, 33), (131, 1), (145, 8),
+                                 (209, 16), (224, 4), (225, 16), (233, 20), (238, 9), (239, 16), (256, 3)])
+def test_factor_path_edges(hsi, orc, B, T):
+    """Band counts at the ends of every path (tiles to 124, blocked to 128, in place to
+    238, workspace above), rows that do and do not fill the groups of four and 32 that
+    the trailing update and the solves take, the targets' stage in the block-row buffer
+    (to 224) and in the diagonal block's place (225 on), several target chunks, and a
+    workspace that starts on 8 bytes only; two frames at once."""
+    sc = hsi.scene(B, n_targets=min(T, 16), target_frac=0.01, frame_seed=B + T)
+    rng = np.random.default_rng(B)
+    lib = rng.uniform(0.05, 1.0, (T, B)).astype(np.float32)
+    hosts = []
+    for k in range(2):
+        sc.frame_seed = 100 * B + k
+        cube, _ = hsi.generate(sc, 48, 64)
+        hosts.append(_download(cube, B, 48 * 64))
+    made = [_fp64_moments_on_device(orc, h) for h in hosts]
+    gm = torch.stack([m for m, _ in made]).contiguous()
+    n = hsi.statistics_elements(B, T)
+    s64 = torch.full((2, n), np.nan, dtype=torch.float64, device="cuda")
+    status = torch.full((2,), -1, dtype=torch.int32, device="cuda")
+    L = hsi.lib()
+    wsb = L.hsi_factor_workspace_bytes(2, B)
+    ws = torch.empty(wsb + 8, dtype=torch.uint8, device="cuda")[8:]
+    tg = torch.from_numpy(lib).cuda()
+    p = lambda t: t.data_ptr()  # noqa: E731
+    hsi.check(L.hsi_build_statistics(2, B, T, 1e-5, p(gm), p(tg), 0, p(s64), None, None, p(status), p(ws), wsb, None))
+    torch.cuda.synchronize()
+    for k in range(2):
+        assert int(status[k]) == 0
+        st, want = orc.build_statistics(*made[k][1], lib, 1e-5)
+        assert st == 0
+        got = hsi.unpack_statistics(s64[k].cpu().numpy(), B, T)
+        for name in ("mean", "whitener", "target_white", "target_norm2", "cem_weight"):
+            err = np.max(np.abs(got[name] - want[name])) / max(np.max(np.abs(want[name])), 1e-30)
+            assert err < 1e-9, f"{name}: {err:.3e}"
+        assert np.all(np.triu(got["whitener"], 1) == 0)
+
+
 def test_factor_against_reference_fixtures(hsi, golden):
     for prefix in ("stats", "b113"):
         g = lambda k: golden[f"{prefix}_{k}"]  # noqa: E731

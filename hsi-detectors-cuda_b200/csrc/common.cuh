@@ -13,11 +13,17 @@
 
 namespace hsi_b200 {
 
-// Largest number of try_wait polls a pipeline wait makes before it gives up,
-// records HSI_E_TIMEOUT and lets the kernel unwind.  Each poll suspends for a
-// hardware-chosen interval, so this is seconds of wall time: far beyond any
+// Largest number of polls a wait makes before it gives up, records
+// HSI_E_TIMEOUT and lets the kernel unwind: seconds of wall time, far beyond any
 // legitimate wait, short enough that a broken pipeline returns an error.
-constexpr uint32_t kWaitLimit = 1u << 26;
+constexpr uint32_t kWaitLimit = 1u << 26;  // polls of a flag in memory
+// Polls of an mbarrier.  Each may suspend the warp for up to kWaitNs (it wakes
+// when the phase completes).  Without the hint a poll came back after a few
+// cycles, and the waiting warps of the warp-specialised kernels took issue
+// slots from the working ones: RX/ACE on the tensor cores (2048 x 1024 x 113) 375 us,
+// 348 us with it; the screen's logits (2048 x 2048 x 224) 464 us and 451 us.
+constexpr uint32_t kMbarPolls = 1u << 22;
+constexpr uint32_t kWaitNs = 1000;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -50,18 +56,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity)
+      : "r"(smem_addr(bar)), "r"(parity), "r"(kWaitNs)
       : "memory");
   return done != 0;
 }
 
-// Wait for phase `parity` of `bar` to complete, polling at most kWaitLimit
+// Wait for phase `parity` of `bar` to complete, polling at most kMbarPolls
 // times.  Returns false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kWaitLimit; ++i) {
+  for (uint32_t i = 0; i < kMbarPolls; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
   }
   return false;

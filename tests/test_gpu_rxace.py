@@ -112,6 +112,42 @@ def test_plain_path_group_and_tile_edges(hsi, orc, B, T, dtype, H, W, off):
     _check_scores(orc, host, S, rx.cpu().numpy(), ace.cpu().numpy(), at.cpu().numpy(), maps.cpu().numpy(), T)
 
 
+@pytest.mark.parametrize("B,T", [(1, 0), (1, 16), (8, 5), (16, 16), (17, 16), (31, 1), (32, 8), (33, 2), (56, 9),
+                                 (64, 16), (65, 3), (80, 16), (96, 7), (97, 16), (112, 16), (125, 3), (127, 2)])
+@pytest.mark.parametrize("dtype,H,W", [(0, 9, 71), (1, 8, 8), (1, 163, 151), (0, 1, 1)])
+def test_tensor_path_steps_and_rounds(hsi, orc, B, T, dtype, H, W):
+    """Every count of 32-band steps and their edges, targets among the rows of the
+    first and the second round and of both row halves, one and several target
+    passes, rings of two to eight boxes, one to many tiles per block, ragged ends.
+    Columns past the frame hold NaN and are never scored."""
+    P = H * W
+    rng = np.random.default_rng(1000 * B + 10 * T + H)
+    mix = rng.standard_normal((B, min(B, 6)))
+    many = 4 * B + 200
+    back = (mix @ rng.standard_normal((mix.shape[1], many + P)) * 0.1 + 0.5
+            + 0.02 * rng.standard_normal((B, many + P))).astype(np.float32)
+    lib = (0.5 + 0.1 * rng.standard_normal((T, B))).astype(np.float32)
+    S = _fp64_stats(orc, np.ascontiguousarray(back[:, :many]), lib, 1e-5)
+    stats = torch.from_numpy(_pack(S)).cuda()
+    tdt = torch.float32 if dtype == 0 else torch.float16
+    stride = (P + 7) // 8 * 8
+    cube = torch.full((B, stride), float("nan"), dtype=tdt, device="cuda")
+    cube[:, :P] = torch.from_numpy(back[:, many:].copy()).cuda().to(tdt)
+    rx = torch.full((P,), np.nan, device="cuda")
+    ace = torch.full((P,), np.nan, device="cuda") if T else None
+    at = torch.full((P,), -9, dtype=torch.int32, device="cuda") if T else None
+    maps = torch.full((max(T, 1), P), np.nan, device="cuda")
+    hsi.rx_ace(cube, H, W, B, stats, T, dtype=dtype, rx=rx, ace_best=ace, ace_target=at,
+               ace_maps=maps if T else None, simt=False)
+    torch.cuda.synchronize()
+    host = cube[:, :P].float().cpu().numpy()
+    if T == 0:
+        rx0 = orc.rx(host, S)
+        assert np.max(np.abs(rx.cpu().numpy() - rx0) / np.maximum(1.0, np.abs(rx0))) <= TOL
+        return
+    _check_scores(orc, host, S, rx.cpu().numpy(), ace.cpu().numpy(), at.cpu().numpy(), maps.cpu().numpy(), T)
+
+
 @pytest.mark.parametrize("dtype", [0, 1])
 def test_rx_ace_tensor_core_at_size(hsi, orc, dtype):
     """512 x 512 x 113 with anomalies, 8 targets, both cube types: the tensor-core

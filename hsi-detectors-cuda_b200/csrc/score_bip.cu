@@ -5,9 +5,18 @@
 // (src/sam.cu:281-309).  Here the transpose is fused into the scoring pass:
 // the cube crosses HBM once, and no BSQ scratch copy exists.
 //
-// Each warp takes tiles of 32 pixels on its own, as a two-step software
-// pipeline: while it scores one tile from shared memory, 16-byte cp.async
-// copies bring the next.  A tile's 32 * B floats are contiguous in BIP and are
+// Each warp takes tiles of 32 pixels on its own: 16-byte cp.async copies bring a
+// tile and the warp scores it from shared memory, while the block's other warps
+// are at other stages.  One buffer a warp and as many warps as shared memory
+// holds (up to 16 a block) keep more of both going than two buffers and half the
+// warps: 1024 x 1024 x 113 with 8 targets 101 us, 140 us with two; at 224 bands
+// 237 us and 660 us.  The next tile's copies start when the last target group has
+// read this one and run under the angles.  Rows of up to some 50 bands leave room
+// for two buffers in many warps, whose copies then run under the products too
+// (1024 x 1024 x 16 with 8 targets 33 us, 37 us with one).  At 113 bands shared
+// memory bounds the kernel: a band of a tile is one wavefront in, one out and four
+// for the broadcast target bank.
+// A tile's rows of B floats are contiguous in BIP and are
 // scored where they land, with no transpose: lane p reads its own pixel's row,
 // p * S floats into the tile, V bands at a time.  The row stride S and the read
 // width V make those reads free of bank conflicts -- V = 1 for an odd band
@@ -20,8 +29,7 @@
 // best angles and best targets are bit-identical to scoring the transposed
 // cube.  All targets are scored from shared memory in one pass over HBM
 // (groups of 8 or 16, two targets per packed FMA, the bank zero-padded to the
-// group).  A block holds as many warps as shared memory allows, up to 8, and
-// one copy of the target bank.
+// group).
 #include "common.cuh"
 #include "launch_state.h"
 #include "sam_math.cuh"
@@ -30,7 +38,8 @@ namespace hsi_b200 {
 namespace {
 
 constexpr int kPx = 32;          // pixels per warp tile
-constexpr int kMaxWarps = 8;     // warps per block
+// warps per block, at most: with two tile buffers a warp and with one
+__host__ __device__ constexpr int max_warps(bool two) { return two ? 8 : 16; }
 constexpr int kMaxTargets = 64;
 constexpr size_t kSmemCap = 227 * 1024;
 
@@ -57,11 +66,11 @@ __host__ __device__ inline int padded_targets(int targets) {
   const int g = group_of(targets);
   return (targets + g - 1) / g * g;
 }
-// bytes of the bank [b][padded targets], the target scales and `warps` double-buffered tiles
+// bytes of the bank [b][padded targets] and the target scales; of a tile
 __host__ __device__ inline size_t bip_fixed_bytes(int bands, int targets) {
   return sizeof(float) * (static_cast<size_t>(bands) * padded_targets(targets) + kMaxTargets);
 }
-__host__ __device__ inline size_t bip_warp_bytes(int bands) { return sizeof(float) * 2 * tile_floats(bands); }
+__host__ __device__ inline size_t bip_warp_bytes(int bands) { return sizeof(float) * tile_floats(bands); }
 
 __device__ __forceinline__ void cp_async16(void* dst, const void* src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(dst)), "l"(src) : "memory");
@@ -83,9 +92,16 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int npx,
     for (int e = 4 * n4 + lane; e < n; e += 32) dst[e] = __ldg(src + e);
   } else if (aligned) {  // B = 0 mod 8: whole 16-byte chunks, re-strided per pixel
     const int q = B / 4;
+    const int rows = 32 / q, rest = 32 - rows * q;  // a step of 32 chunks in pixels and chunks
+    int p = lane / q, c = lane - p * q;
     for (int i = lane; i < npx * q; i += 32) {
-      const int p = i / q;
-      cp_async16(dst + p * S + 4 * (i - p * q), src + 4 * i);
+      cp_async16(dst + p * S + 4 * c, src + 4 * i);
+      p += rows;
+      c += rest;
+      if (c >= q) {
+        c -= q;
+        ++p;
+      }
     }
     cp_async_commit();
   } else {
@@ -101,7 +117,7 @@ __device__ __forceinline__ void load_tile(float* dst, const float* src, int npx,
 template <int G, int V, bool kNorm>
 __device__ __forceinline__ void band_loop(const float* xr, const float* tgc, int TP, int B, float2 (&acc)[G / 2],
                                           float& nrm) {
-#pragma unroll 2
+#pragma unroll(8 / V)
   for (int b = 0; b < B; b += V) {
     float x[V];
     if constexpr (V == 4) {
@@ -128,22 +144,15 @@ __device__ __forceinline__ void band_loop(const float* xr, const float* tgc, int
   }
 }
 
-template <int G, int V>
-__global__ void __launch_bounds__(kMaxWarps * 32) sam_bip_kernel(const BipArgs a) {
+// kTwo: two tile buffers a warp.
+template <int G, int V, bool kTwo>
+__global__ void __launch_bounds__(max_warps(kTwo) * 32, !kTwo ? 1 : G == 8 ? 4 : 3) sam_bip_kernel(const BipArgs a) {
   extern __shared__ __align__(16) float sm[];
   const int B = a.bands, T = a.targets, TP = (T + G - 1) / G * G, S = row_stride(B);
   float* tg = sm;                  // [b][TP], zero beyond T
   float* scale = tg + B * TP;      // [t] = 1 / |r_t| (0 for a zero target)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, warps = blockDim.x >> 5;
-  const int tf = tile_floats(B);
-  float* buf = scale + kMaxTargets + static_cast<size_t>(warp) * 2 * tf;  // two tiles [p][S]
-  for (int i = threadIdx.x; i < B * TP; i += blockDim.x) {
-    const int b = i / TP, t = i - b * TP;
-    tg[i] = t < T ? a.lib[static_cast<int64_t>(t) * B + b] : 0.0f;
-  }
-  for (int t = threadIdx.x; t < T; t += blockDim.x) scale[t] = a.norms[t] > 0.0f ? 1.0f / a.norms[t] : 0.0f;
-  __syncthreads();
-
+  float* buf = scale + kMaxTargets + static_cast<size_t>(warp) * (kTwo ? 2 : 1) * tile_floats(B);  // tiles [p][S]
   const int64_t ntiles = div_up<int64_t>(a.pixels, kPx);
   const int64_t step = static_cast<int64_t>(gridDim.x) * warps;
   int64_t tile = static_cast<int64_t>(blockIdx.x) * warps + warp;
@@ -152,18 +161,28 @@ __global__ void __launch_bounds__(kMaxWarps * 32) sam_bip_kernel(const BipArgs a
     return static_cast<int>(left < kPx ? left : kPx);
   };
   if (tile < ntiles) load_tile(buf, a.cube + tile * kPx * B, npx_of(tile), B, S, lane, a.aligned);
+  for (int i = threadIdx.x; i < B * TP; i += blockDim.x) {
+    const int b = i / TP, t = i - b * TP;
+    tg[i] = t < T ? a.lib[static_cast<int64_t>(t) * B + b] : 0.0f;
+  }
+  for (int t = threadIdx.x; t < T; t += blockDim.x) scale[t] = a.norms[t] > 0.0f ? 1.0f / a.norms[t] : 0.0f;
+  __syncthreads();
+
   for (int it = 0; tile < ntiles; tile += step, ++it) {
-    const float* cur = buf + (it & 1) * tf;
     const int npx = npx_of(tile);
+    const int64_t next = tile + step;
     cp_async_wait_all();
     __syncwarp();
-    // the next tile's copies run while this one is scored
-    const int64_t next = tile + step;
-    if (next < ntiles) load_tile(buf + ((it + 1) & 1) * tf, a.cube + next * kPx * B, npx_of(next), B, S, lane,
-                                 a.aligned);
-    if (lane < npx) {
-      const int64_t px = tile * kPx + lane;
-      const float* xr = cur + lane * S;
+    float* other = buf;
+    if constexpr (kTwo) {
+      other = scale + kMaxTargets + static_cast<size_t>(2 * warp + (~it & 1)) * tile_floats(B);
+      if (next < ntiles) load_tile(other, a.cube + next * kPx * B, npx_of(next), B, S, lane, a.aligned);
+    }
+    const bool in = lane < npx;  // a ragged last tile's other lanes repeat its first pixel
+    const int64_t px = tile * kPx + lane;
+    const float* xr = buf + (in ? lane * S : 0);
+    if (!kTwo || in) {
+      const bool store = kTwo || in;
       float nrm = 0.0f, rn = 0.0f, best = -2.0f;
       int32_t best_t = -1;
       for (int t0 = 0; t0 < T; t0 += G) {
@@ -176,6 +195,10 @@ __global__ void __launch_bounds__(kMaxWarps * 32) sam_bip_kernel(const BipArgs a
           rn = nrm > 0.0f ? rsqrtf(nrm) : 0.0f;
         } else {
           band_loop<G, V, false>(xr, tg + t0, TP, B, acc, nrm);
+        }
+        if (!kTwo && t0 + G >= T && next < ntiles) {
+          __syncwarp();  // every lane is done with the tile: the next one arrives under the angles
+          load_tile(buf, a.cube + next * kPx * B, npx_of(next), B, S, lane, a.aligned);
         }
 #pragma unroll
         for (int k = 0; k < G; k += 2) {
@@ -190,38 +213,61 @@ __global__ void __launch_bounds__(kMaxWarps * 32) sam_bip_kernel(const BipArgs a
             best = c1;
             best_t = t0 + k + 1;
           }
-          if (a.maps) {
+          if (a.maps && store) {
             const float2 ang = angle_of_cos2(make_float2(c0, c1));
             a.maps[static_cast<int64_t>(t0 + k) * a.map_stride + px] = ang.x;
             if (k + 1 < nt) a.maps[static_cast<int64_t>(t0 + k + 1) * a.map_stride + px] = ang.y;
           }
         }
       }
-      if (a.best) a.best[px] = angle_of_cos(best);
-      if (a.best_t) a.best_t[px] = best_t;
+      if (a.best && store) a.best[px] = angle_of_cos(best);
+      if (a.best_t && store) a.best_t[px] = best_t;
     }
-    __syncwarp();  // every lane is done with cur before the next round's copies refill it
+    if constexpr (kTwo) {
+      __syncwarp();  // every lane is done with the tile before the next round's copies refill it
+      buf = other;
+    }
   }
   cp_async_wait_all();  // never leave copies in flight into shared memory
 }
 
-template <int G, int V>
-int launch_bip(const BipArgs& a, cudaStream_t stream) {
-  const size_t fixed = bip_fixed_bytes(a.bands, a.targets), per_warp = bip_warp_bytes(a.bands);
-  if (fixed + per_warp > kSmemCap) return HSI_E_CAPACITY;
+template <int G, int V, bool kTwo>
+int launch_bip_k(const BipArgs& a, cudaStream_t stream) {
+  const size_t fixed = bip_fixed_bytes(a.bands, a.targets), per_warp = bip_warp_bytes(a.bands) * (kTwo ? 2 : 1);
   const int64_t ntiles = div_up<int64_t>(a.pixels, kPx);
-  int warps = static_cast<int>((kSmemCap - fixed) / per_warp);
-  if (warps > kMaxWarps) warps = kMaxWarps;
-  if (warps > ntiles) warps = static_cast<int>(ntiles);
+  // the block size that keeps most warps on an SM (1 KB of each block's shared memory is the system's)
+  int warps = 1;
+  size_t most = 0;
+  for (int w = max_warps(kTwo); w >= 1; --w) {
+    const size_t block = fixed + w * per_warp;
+    const size_t on_sm = block > kSmemCap ? 0 : w * ((kSmemCap + 1024) / (block + 1024));
+    if (on_sm > most) {
+      most = on_sm;
+      warps = w;
+    }
+  }
+  // few tiles: over all SMs, but four warps a block share the staging of the bank
+  const int64_t over_sms = div_up<int64_t>(ntiles, device_sm_count());
+  const int64_t spread = over_sms > 4 ? over_sms : 4;
+  if (warps > spread) warps = static_cast<int>(spread);
   const size_t smem = fixed + static_cast<size_t>(warps) * per_warp;
-  const cudaError_t e = raise_smem_limit(sam_bip_kernel<G, V>, static_cast<int>(smem));
+  const cudaError_t e = raise_smem_limit(sam_bip_kernel<G, V, kTwo>, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  const int per_sm = device_residency(sam_bip_kernel<G, V>, warps * 32, smem);
+  const int per_sm = device_residency(sam_bip_kernel<G, V, kTwo>, warps * 32, smem);
   const int64_t blocks_needed = div_up<int64_t>(ntiles, warps);
   const int64_t wave = static_cast<int64_t>(device_sm_count()) * (per_sm > 0 ? per_sm : 1);
   const int grid = static_cast<int>(blocks_needed < wave ? blocks_needed : wave);
-  sam_bip_kernel<G, V><<<grid, warps * 32, smem, stream>>>(a);
+  sam_bip_kernel<G, V, kTwo><<<grid, warps * 32, smem, stream>>>(a);
   return static_cast<int>(cudaGetLastError());
+}
+
+template <int G, int V>
+int launch_bip(const BipArgs& a, cudaStream_t stream) {
+  const size_t fixed = bip_fixed_bytes(a.bands, a.targets), tile = bip_warp_bytes(a.bands);
+  if (fixed + 2 * tile > kSmemCap) return HSI_E_CAPACITY;
+  // Two buffers while two blocks of eight warps can have them (up to some 50 bands).
+  if (2 * (fixed + 16 * tile + 1024) <= kSmemCap + 1024) return launch_bip_k<G, V, true>(a, stream);
+  return launch_bip_k<G, V, false>(a, stream);
 }
 
 template <int G>

@@ -72,6 +72,15 @@ def test_bip_equals_bsq_bit_for_bit(hsi, orc, H, W, B, T, off):
     assert float(np.abs(best.cpu().numpy() - f64).max()) <= 5e-5
 
 
+@pytest.mark.parametrize("H,W,B,T,off", [(331, 479, 113, 8, 0), (331, 479, 113, 17, 1), (263, 251, 64, 8, 0),
+                                         (263, 251, 224, 9, 0), (263, 251, 250, 40, 0), (600, 523, 16, 16, 0),
+                                         (400, 401, 50, 8, 0), (400, 401, 52, 16, 0), (160, 149, 256, 64, 0)])
+def test_bip_many_tiles_per_warp(hsi, orc, H, W, B, T, off):
+    """Several tiles per warp with one tile buffer (refilled under the angles) and
+    with two, band counts on both sides of that line, the last tile ragged."""
+    test_bip_equals_bsq_bit_for_bit(hsi, orc, H, W, B, T, off)
+
+
 def test_bip_pixel_equal_to_a_target_scores_zero(hsi):
     H, W, B, T = 8, 8, 20, 3
     rng = np.random.default_rng(5)

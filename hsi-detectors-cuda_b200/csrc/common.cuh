@@ -17,13 +17,9 @@ namespace hsi_b200 {
 // HSI_E_TIMEOUT and lets the kernel unwind: seconds of wall time, far beyond any
 // legitimate wait, short enough that a broken pipeline returns an error.
 constexpr uint32_t kWaitLimit = 1u << 26;  // polls of a flag in memory
-// Polls of an mbarrier.  Each may suspend the warp for up to kWaitNs (it wakes
-// when the phase completes).  Without the hint a poll came back after a few
-// cycles, and the waiting warps of the warp-specialised kernels took issue
-// slots from the working ones: RX/ACE on the tensor cores (2048 x 1024 x 113) 375 us,
-// 348 us with it; the screen's logits (2048 x 2048 x 224) 464 us and 451 us.
-constexpr uint32_t kMbarPolls = 1u << 22;
-constexpr uint32_t kWaitNs = 1000;
+// Polls of mbar_wait_idle, each of which may suspend the warp for up to kIdleNs.
+constexpr uint32_t kIdlePolls = 1u << 22;
+constexpr uint32_t kIdleNs = 1000;
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -56,19 +52,40 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   uint32_t done;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
+      "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(done)
-      : "r"(smem_addr(bar)), "r"(parity), "r"(kWaitNs)
+      : "r"(smem_addr(bar)), "r"(parity)
       : "memory");
   return done != 0;
 }
 
-// Wait for phase `parity` of `bar` to complete, polling at most kMbarPolls
+// Wait for phase `parity` of `bar` to complete, polling at most kWaitLimit
 // times.  Returns false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-  for (uint32_t i = 0; i < kMbarPolls; ++i) {
+  for (uint32_t i = 0; i < kWaitLimit; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
+  }
+  return false;
+}
+
+// The same for kernels that are short of issue slots: a poll without the time
+// hint comes back after a few cycles, and the waiting warps take slots from the
+// working ones.  RX/ACE on the tensor cores (2048 x 1024 x 113) 375 us with
+// mbar_wait, 348 us with this; the screen's logits (2048 x 2048 x 224) 464 and
+// 451 us.  Waking costs more: the FP32 scorer, whose consumers wait for every
+// stage, is 2 to 4 % slower with it and keeps mbar_wait.
+__device__ __forceinline__ bool mbar_wait_idle(uint64_t* bar, uint32_t parity) {
+  for (uint32_t i = 0; i < kIdlePolls; ++i) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cta.shared::cta.b64 p, [%1], %2, %3;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(done)
+        : "r"(smem_addr(bar)), "r"(parity), "r"(kIdleNs)
+        : "memory");
+    if (done) return true;
   }
   return false;
 }

@@ -328,7 +328,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (int i = 0; i < 2 * n; ++i) {
         const int s = i & (kIn - 1);
         const uint32_t ph = (i >> in_log) & 1u;
-        if (*abort_flag || !mbar_wait(&in_empty[s], ph ^ 1u)) {
+        if (*abort_flag || !mbar_wait_idle(&in_empty[s], ph ^ 1u)) {
           record_error(args.status, HSI_E_TIMEOUT);
           *abort_flag = 1;
           break;
@@ -341,8 +341,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         parity = (parity & ~(1u << s)) | (ph << s);
       }
       for (int s = 0; s < kIn; ++s)
-        if ((pending >> s) & 1u) mbar_wait(&in_full[s], (parity >> s) & 1u);
-      mbar_wait(w_full, 0);
+        if ((pending >> s) & 1u) mbar_wait_idle(&in_full[s], (parity >> s) & 1u);
+      mbar_wait_idle(w_full, 0);
     }
   } else if (warp == kWarpMma) {
     if (lane == 0) {
@@ -351,14 +351,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       const uint32_t id64 = idesc_s8_s32(kTilePx, 64);    // M2
       const int rounds = args.rows > 32 ? 2 : 1;
       bool issued = false;
-      if (n > 0 && !mbar_wait(w_full, 0)) {
+      if (n > 0 && !mbar_wait_idle(w_full, 0)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
       }
       bool ok = true;
       for (int i = 0; i < n && ok && !*abort_flag; ++i) {
         const int so = i % kOpStages;
-        if (!mbar_wait(&op_full[so], (i / kOpStages) & 1u)) {
+        if (!mbar_wait_idle(&op_full[so], (i / kOpStages) & 1u)) {
           record_error(args.status, HSI_E_TIMEOUT);
           *abort_flag = 1;
           break;
@@ -367,7 +367,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint64_t a0 = smem_desc_sw128(a), a1 = smem_desc_sw128(a + kLimbBytes);
         const uint64_t a2 = smem_desc_sw128(a + 2 * kLimbBytes);
         for (int h = 0; h < rounds; ++h) {
-          if (!mbar_wait(&acc_empty[h], (i & 1u) ^ 1u)) {
+          if (!mbar_wait_idle(&acc_empty[h], (i & 1u) ^ 1u)) {
             record_error(args.status, HSI_E_TIMEOUT);
             *abort_flag = 1;
             ok = false;
@@ -395,7 +395,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
       if (issued) {
         umma_commit(mma_done);
-        if (!mbar_wait(mma_done, 0)) record_error(args.status, HSI_E_TIMEOUT);
+        if (!mbar_wait_idle(mma_done, 0)) record_error(args.status, HSI_E_TIMEOUT);
       }
     }
   } else if (warp < kWarpEpi0) {
@@ -411,7 +411,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     const float4* mu = reinterpret_cast<const float4*>(mean32 + w * kBandStep);
     for (int i = 0; i < n && w < steps; ++i) {
       const int j = 2 * i + half, s = j & (kIn - 1), so = i % kOpStages;
-      if (!mbar_wait(&in_full[s], (j >> in_log) & 1u)) {
+      if (!mbar_wait_idle(&in_full[s], (j >> in_log) & 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;
@@ -454,8 +454,8 @@ __global__ void __launch_bounds__(kThreads, 1)
         mbar_arrive(&in_empty[s]);
         mbar_arrive(&red_bar[half * 2 + (i & 1)]);
       }
-      if (!mbar_wait(&red_bar[half * 2 + (i & 1)], (i >> 1) & 1u) ||
-          !mbar_wait(&op_empty[so], ((i / kOpStages) & 1u) ^ 1u)) {
+      if (!mbar_wait_idle(&red_bar[half * 2 + (i & 1)], (i >> 1) & 1u) ||
+          !mbar_wait_idle(&op_empty[so], ((i / kOpStages) & 1u) ^ 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;
@@ -513,7 +513,7 @@ __global__ void __launch_bounds__(kThreads, 1)
     for (int i = 0; i < n; ++i) {
       const int so = i % kOpStages;
       // the scales were published with the limbs (already complete: the MMA waited on it)
-      if (!mbar_wait(&op_full[so], (i / kOpStages) & 1u)) {
+      if (!mbar_wait_idle(&op_full[so], (i / kOpStages) & 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;
@@ -527,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool mine = hf == 0;  // zzp and zbuf may be written: the last tile's have been read
 #pragma unroll 1
       for (int h = 0; h < rounds && ok; ++h) {
-        if (!mbar_wait(&acc_full[h], i & 1u)) {
+        if (!mbar_wait_idle(&acc_full[h], i & 1u)) {
           ok = false;
           break;
         }
@@ -583,7 +583,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           if (n0 + 8 <= B) {
             block(std::true_type{}, n0, v);
           } else {
-            if (!mine && !mbar_wait(&half_empty[q], (i & 1u) ^ 1u)) {
+            if (!mine && !mbar_wait_idle(&half_empty[q], (i & 1u) ^ 1u)) {
               ok = false;
               break;
             }
@@ -595,14 +595,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         __syncwarp();
         if (lane == 0) mbar_arrive(&acc_empty[h]);
       }
-      if (ok && !mine) ok = mbar_wait(&half_empty[q], (i & 1u) ^ 1u);
+      if (ok && !mine) ok = mbar_wait_idle(&half_empty[q], (i & 1u) ^ 1u);
       if (ok && hf == 1) {
         zzp[px] = zz;
         __syncwarp();
         if (lane == 0) mbar_arrive(&half_full[q]);
         continue;
       }
-      if (!ok || !mbar_wait(&half_full[q], i & 1u)) {
+      if (!ok || !mbar_wait_idle(&half_full[q], i & 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;

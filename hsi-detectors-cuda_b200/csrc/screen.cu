@@ -661,7 +661,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
       for (int i = 0; i < n; ++i) {
         const int s = i % kIn;
         const uint32_t ph = (i / kIn) & 1u;
-        if (*abort_flag || !mbar_wait(&in_empty[s], ph ^ 1u)) {
+        if (*abort_flag || !mbar_wait_idle(&in_empty[s], ph ^ 1u)) {
           record_error(args.status, HSI_E_TIMEOUT);
           *abort_flag = 1;
           break;
@@ -675,15 +675,15 @@ __global__ void __launch_bounds__(kScrThreads, 1)
         parity = (parity & ~(1u << s)) | (ph << s);
       }
       for (int s = 0; s < kIn; ++s)
-        if ((pending >> s) & 1u) mbar_wait(&in_full[s], (parity >> s) & 1u);
-      mbar_wait(w_full, 0);
+        if ((pending >> s) & 1u) mbar_wait_idle(&in_full[s], (parity >> s) & 1u);
+      mbar_wait_idle(w_full, 0);
     }
   } else if (warp == 1) {
     if (lane == 0) {
       const uint32_t id1 = idesc_f16_amn(kScrTile, kH1);
       const uint32_t id2 = idesc_bf16_f32(kScrTile, kH2);
       bool issued = false;
-      if (n > 0 && !mbar_wait(w_full, 0)) {
+      if (n > 0 && !mbar_wait_idle(w_full, 0)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
       }
@@ -691,7 +691,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
       // layer 2 of tile j
       auto layer2 = [&](int j) -> bool {
         const int pb = j & 1;
-        if (!mbar_wait(&h1_full[pb], (j >> 1) & 1u) || !mbar_wait(acc2_empty, (j & 1u) ^ 1u)) return false;
+        if (!mbar_wait_idle(&h1_full[pb], (j >> 1) & 1u) || !mbar_wait_idle(acc2_empty, (j & 1u) ^ 1u)) return false;
         tc_fence_after();
         const uint64_t dh = smem_desc_sw128(h1 + pb * kScrTile * 128);
 #pragma unroll
@@ -702,7 +702,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
       };
       for (int i = 0; i < n && !*abort_flag; ++i) {
         const int s = i % kIn, pb = i & 1;
-        if (!mbar_wait(&in_full[s], (i / kIn) & 1u) || !mbar_wait(&acc1_empty[pb], ((i >> 1) & 1u) ^ 1u)) {
+        if (!mbar_wait_idle(&in_full[s], (i / kIn) & 1u) || !mbar_wait_idle(&acc1_empty[pb], ((i >> 1) & 1u) ^ 1u)) {
           record_error(args.status, HSI_E_TIMEOUT);
           *abort_flag = 1;
           break;
@@ -729,7 +729,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
       }
       if (issued) {
         umma_commit(mma_done);
-        if (!mbar_wait(mma_done, 0)) record_error(args.status, HSI_E_TIMEOUT);
+        if (!mbar_wait_idle(mma_done, 0)) record_error(args.status, HSI_E_TIMEOUT);
       }
     }
   } else {
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
     const float b3 = w3[kH2];
     for (int i = 0; i < n; ++i) {
       const int pb = i & 1;
-      if (!mbar_wait(&acc1_full[pb], (i >> 1) & 1u)) {
+      if (!mbar_wait_idle(&acc1_full[pb], (i >> 1) & 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;
@@ -772,7 +772,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
         const __nv_bfloat162 v2 = __floats2bfloat162_rn(a0, a1);
         packed[16 + j] = *reinterpret_cast<const uint32_t*>(&v2);
       }
-      if (!mbar_wait(&h1_empty[pb], ((i >> 1) & 1u) ^ 1u)) {
+      if (!mbar_wait_idle(&h1_empty[pb], ((i >> 1) & 1u) ^ 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(kScrThreads, 1)
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) mbar_arrive(&h1_full[pb]);
-      if (!mbar_wait(acc2_full, i & 1u)) {
+      if (!mbar_wait_idle(acc2_full, i & 1u)) {
         record_error(args.status, HSI_E_TIMEOUT);
         *abort_flag = 1;
         break;

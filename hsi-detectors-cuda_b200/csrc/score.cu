@@ -35,6 +35,10 @@ constexpr int kTile = kGroupThreads * kPPT;
 // (twice the warps of one warpgroup at four pixels, for the same tile).
 constexpr int kFusedThreads = 256;
 constexpr int kFusedPPT = kTile / kFusedThreads;
+// The wide form of the same: four pixels per thread in seven warps (with the
+// producer 16 warps of two CTAs an SM, 128 registers each), tiles of 896 pixels.
+constexpr int kWidePPT = 4;
+constexpr int kWideThreads = 224;
 constexpr int kMaxTableFrames = 256;
 constexpr int kFiltersPerPass = HSI_MAX_FILTERS_PER_PASS;
 constexpr int kMaxInline = 64;  // frames whose descriptors travel inside one launch
@@ -54,12 +58,16 @@ struct CubeTraits<float> {
   static constexpr int kStageBands = 16;  // band planes of a tile per stage
   static constexpr int kStages = 3;
   static constexpr int kStagesFused = 2;
+  static constexpr int kStageBandsWide = 8;
+  static constexpr int kStagesWide = 3;
 };
 template <>
 struct CubeTraits<__half> {
   static constexpr int kStageBands = 8;
   static constexpr int kStages = 10;
   static constexpr int kStagesFused = 7;
+  static constexpr int kStageBandsWide = 4;  // FP16 frames take the narrow form
+  static constexpr int kStagesWide = 3;
 };
 
 struct ScoreParams {
@@ -131,10 +139,23 @@ struct SmemLayout {
   size_t stage_bytes, filt_off, scale_off, bar_off, prefix_off, total;
 };
 
-template <typename T>
+template <bool kWide>
+constexpr int tile_px() {
+  return kWide ? kWideThreads * kWidePPT : kTile;
+}
+template <bool kWide>
+constexpr int fused_threads() {
+  return kWide ? kWideThreads : kFusedThreads;
+}
+template <typename T, bool kWide>
+constexpr int stage_bands() {
+  return kWide ? CubeTraits<T>::kStageBandsWide : CubeTraits<T>::kStageBands;
+}
+
+template <typename T, bool kWide>
 __host__ __device__ inline SmemLayout smem_layout(int groups, int max_bands, int slots, int stages) {
   SmemLayout l;
-  l.stage_bytes = static_cast<size_t>(CubeTraits<T>::kStageBands) * kTile * sizeof(T);
+  l.stage_bytes = static_cast<size_t>(stage_bands<T, kWide>()) * tile_px<kWide>() * sizeof(T);
   size_t off = l.stage_bytes * stages;
   l.filt_off = off;
   off += static_cast<size_t>(groups) * max_bands * slots * sizeof(float);
@@ -422,42 +443,61 @@ __device__ __forceinline__ void consumer_loop(const ScoreParams& prm, const int*
 // thread keep the accumulators at 2 * (KS + KC) registers, so 256 consumer
 // threads fit per CTA at three CTAs per SM (twice the warps of one warpgroup
 // at four pixels per thread, to hide the shared-memory and FMA latencies).
-template <typename T, int K, bool kNorm>
+// With 16 filters the bank's broadcast reads are eight of the ten shared-memory
+// wavefronts of a band and 64 pixels and hold the kernel (66 % of its cycles, the
+// FMA pipe 55 %): the wide form gives each thread four pixels, six wavefronts for
+// as many pixels, in seven warps at two CTAs per SM.
+template <typename T, int K, bool kNorm, bool kWide>
 __device__ __forceinline__ void consume_stage_fused(const T* stage, const float* filt, int nb, int tid,
-                                                    float2 (&acc)[K / 2][kFusedPPT], float2& nrm) {
-  static_assert(kFusedPPT == 2, "two pixels per fused consumer thread");
+                                                    float2 (&acc)[K / 2][kWide ? kWidePPT : kFusedPPT],
+                                                    float2 (&nrm)[kWide ? 2 : 1]) {
   static_assert(K % 4 == 0, "filters in groups of four");
-  const T* src = stage + tid * kFusedPPT;
+  constexpr int PPT = kWide ? kWidePPT : kFusedPPT;
+  const T* src = stage + tid * PPT;
   auto band = [&](int i) {
-    const float2 v = load2<T>(src + i * kTile);
-    if constexpr (kNorm) nrm = ffma2(v, v, nrm);
-    const float2 d0 = make_float2(v.x, v.x), d1 = make_float2(v.y, v.y);
+    float x[PPT];
+    if constexpr (kWide) {
+      load4<T>(src + i * tile_px<kWide>(), x);
+    } else {
+      const float2 v = load2<T>(src + i * tile_px<kWide>());
+      x[0] = v.x;
+      x[1] = v.y;
+    }
+    if constexpr (kNorm) {
+#pragma unroll
+      for (int j = 0; j < PPT; j += 2) {
+        const float2 v = make_float2(x[j], x[j + 1]);
+        nrm[j / 2] = ffma2(v, v, nrm[j / 2]);
+      }
+    }
     const float* fr = filt + i * K;
 #pragma unroll
     for (int k = 0; k < K; k += 4) {
       const float4 f = ld_shared_f4(fr + k);  // (f_k, f_k+1, f_k+2, f_k+3)
       const float2 fa = make_float2(f.x, f.y), fb = make_float2(f.z, f.w);
-      acc[k / 2][0] = ffma2(d0, fa, acc[k / 2][0]);
-      acc[k / 2][1] = ffma2(d1, fa, acc[k / 2][1]);
-      acc[k / 2 + 1][0] = ffma2(d0, fb, acc[k / 2 + 1][0]);
-      acc[k / 2 + 1][1] = ffma2(d1, fb, acc[k / 2 + 1][1]);
+#pragma unroll
+      for (int j = 0; j < PPT; ++j) acc[k / 2][j] = ffma2(make_float2(x[j], x[j]), fa, acc[k / 2][j]);
+#pragma unroll
+      for (int j = 0; j < PPT; ++j) acc[k / 2 + 1][j] = ffma2(make_float2(x[j], x[j]), fb, acc[k / 2 + 1][j]);
     }
   };
-  if (nb == CubeTraits<T>::kStageBands) {
-#pragma unroll
-    for (int i = 0; i < CubeTraits<T>::kStageBands; ++i) band(i);
+  if (nb == stage_bands<T, kWide>()) {
+    // two bands of four pixels at a time: the wide form has no registers for more
+#pragma unroll(kWide ? 2 : stage_bands<T, kWide>())
+    for (int i = 0; i < stage_bands<T, kWide>(); ++i) band(i);
   } else {
     for (int i = 0; i < nb; ++i) band(i);
   }
 }
 
-template <typename T, int KS, int KC, int kStages>
+template <typename T, int KS, int KC, int kStages, bool kWide>
 __device__ __forceinline__ void consumer_loop_fused(const ScoreParams& prm, const int* prefix, int total_tiles,
                                                     unsigned char* smem, size_t stage_bytes, uint64_t* full,
                                                     uint64_t* empty, volatile int* abort_flag, float* filt,
                                                     float* scale, int tid, int lane) {
   constexpr int K = KS + KC;
-  constexpr int PPT = kFusedPPT;
+  constexpr int PPT = kWide ? kWidePPT : kFusedPPT;
+  constexpr int kStageBands = stage_bands<T, kWide>();
   const int nframes = prm.num_frames;
   int cur_frame = -1;
   int n_s = 0, n_c = 0;
@@ -469,11 +509,11 @@ __device__ __forceinline__ void consumer_loop_fused(const ScoreParams& prm, cons
     const hsi_frame& F = frame_at(prm, f);
     const int B = F.bands;
     if (f != cur_frame) {
-      named_sync(1, kFusedThreads);
+      named_sync(1, fused_threads<kWide>());
       n_s = pass_count(F.num_sam, prm.pass);
       n_c = pass_count(F.num_cem, prm.pass);
       const int t0 = prm.pass * kFiltersPerPass;
-      for (int i = tid; i < B * K; i += kFusedThreads) {
+      for (int i = tid; i < B * K; i += fused_threads<kWide>()) {
         const int b = i / K, k = i % K;
         float v = 0.0f;
         if (k < KS) {
@@ -487,22 +527,24 @@ __device__ __forceinline__ void consumer_loop_fused(const ScoreParams& prm, cons
         const float nrm = tid < n_s ? F.sam_norms[t0 + tid] : 0.0f;
         scale[tid] = nrm > 0.0f ? 1.0f / nrm : 0.0f;
       }
-      named_sync(1, kFusedThreads);
+      named_sync(1, fused_threads<kWide>());
       cur_frame = f;
     }
     const int64_t P = static_cast<int64_t>(F.height) * F.width;
-    const int64_t p0 = static_cast<int64_t>(tile - prefix[f]) * kTile;
+    const int64_t p0 = static_cast<int64_t>(tile - prefix[f]) * tile_px<kWide>();
     const bool active = n_s > 0 || n_c > 0;
 
     float2 acc[K / 2][PPT];
-    float2 nrm = make_float2(0.0f, 0.0f);
+    float2 nrm[kWide ? 2 : 1];
+#pragma unroll
+    for (int j = 0; j < PPT / 2; ++j) nrm[j] = make_float2(0.0f, 0.0f);
 #pragma unroll
     for (int k = 0; k < K / 2; ++k)
 #pragma unroll
       for (int j = 0; j < PPT; ++j) acc[k][j] = make_float2(0.0f, 0.0f);
 
-    for (int b0 = 0; b0 < B; b0 += CubeTraits<T>::kStageBands) {
-      const int nb = B - b0 < CubeTraits<T>::kStageBands ? B - b0 : CubeTraits<T>::kStageBands;
+    for (int b0 = 0; b0 < B; b0 += kStageBands) {
+      const int nb = B - b0 < kStageBands ? B - b0 : kStageBands;
       const int slot = static_cast<int>(it % kStages);
       const uint32_t round = it / kStages;
       if (!aborted && !mbar_wait(&full[slot], round & 1u)) {
@@ -512,7 +554,7 @@ __device__ __forceinline__ void consumer_loop_fused(const ScoreParams& prm, cons
       }
       if (active && !aborted) {
         const T* stage = reinterpret_cast<const T*>(smem + slot * stage_bytes);
-        consume_stage_fused<T, K, (KS > 0)>(stage, filt + b0 * K, nb, tid, acc, nrm);
+        consume_stage_fused<T, K, (KS > 0), kWide>(stage, filt + b0 * K, nb, tid, acc, nrm);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(&empty[slot]);
@@ -530,7 +572,9 @@ __device__ __forceinline__ void consumer_loop_fused(const ScoreParams& prm, cons
             for (int k = 0; k < KS; ++k)
 #pragma unroll
               for (int j = 0; j < PPT; ++j) a[k][j] = (k & 1) ? acc[k / 2][j].y : acc[k / 2][j].x;
-            const float n[PPT] = {nrm.x, nrm.y};
+            float n[PPT];
+#pragma unroll
+            for (int j = 0; j < PPT; ++j) n[j] = (j & 1) ? nrm[j / 2].y : nrm[j / 2].x;
             sam_epilogue<KS, PPT>(F, prm.pass, n_s, p, valid, a, n, scale);
           }
         }
@@ -568,9 +612,9 @@ template <int KS, int KC>
 constexpr int score_groups() {
   return fused_banks<KS, KC>() ? 1 : (KS > 0) + (KC > 0);
 }
-template <int KS, int KC>
+template <int KS, int KC, bool kWide>
 constexpr int consumer_threads() {
-  return fused_banks<KS, KC>() ? kFusedThreads : score_groups<KS, KC>() * kGroupThreads;
+  return fused_banks<KS, KC>() ? fused_threads<kWide>() : score_groups<KS, KC>() * kGroupThreads;
 }
 // Filter slots per band per group in shared memory (duplicated pairs in the
 // two-group layout, plain in the fused one).
@@ -579,19 +623,20 @@ constexpr int score_slots() {
   return fused_banks<KS, KC>() ? KS + KC : 2 * (KS > KC ? KS : KC);
 }
 
-template <typename T, int KS, int KC>
+template <typename T, int KS, int KC, bool kWide>
 constexpr int score_stages() {
-  return fused_banks<KS, KC>() ? CubeTraits<T>::kStagesFused : CubeTraits<T>::kStages;
+  return kWide ? CubeTraits<T>::kStagesWide : fused_banks<KS, KC>() ? CubeTraits<T>::kStagesFused : CubeTraits<T>::kStages;
 }
 
-template <typename T, int KS, int KC>
-__global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<KS, KC>() ? 3 : 1)
+template <typename T, int KS, int KC, bool kWide>
+__global__ void __launch_bounds__(consumer_threads<KS, KC, kWide>() + 32, kWide ? 2 : fused_banks<KS, KC>() ? 3 : 1)
     score_kernel(const __grid_constant__ ScoreParams prm, int max_bands) {
   constexpr int kGroups = score_groups<KS, KC>();
-  constexpr int kStages = score_stages<T, KS, KC>();
+  constexpr int kStages = score_stages<T, KS, KC, kWide>();
   constexpr int kSlots = score_slots<KS, KC>();
+  constexpr int kTilePx = tile_px<kWide>(), kStageBands = stage_bands<T, kWide>();
   extern __shared__ __align__(128) unsigned char smem[];
-  const SmemLayout L = smem_layout<T>(kGroups, max_bands, kSlots, kStages);
+  const SmemLayout L = smem_layout<T, kWide>(kGroups, max_bands, kSlots, kStages);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L.bar_off);
   uint64_t* empty = full + kStages;
   int* prefix = reinterpret_cast<int*>(smem + L.prefix_off);
@@ -609,14 +654,14 @@ __global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<K
                     F.plane_stride >= P && (F.plane_stride & 7) == 0;
     if (!ok && blockIdx.x == 0) record_error(prm.status, HSI_E_INVALID);
     const bool any = ok && (pass_count(F.num_sam, prm.pass) > 0 || pass_count(F.num_cem, prm.pass) > 0);
-    prefix[f + 1] = any ? static_cast<int>(div_up<int64_t>(P, kTile)) : 0;
+    prefix[f + 1] = any ? static_cast<int>(div_up<int64_t>(P, kTilePx)) : 0;
   }
   if (threadIdx.x == 0) {
     prefix[0] = 0;
     *abort_flag = 0;
     for (int s = 0; s < kStages; ++s) {
       mbar_init(&full[s], 1);
-      mbar_init(&empty[s], consumer_threads<KS, KC>() / 32);
+      mbar_init(&empty[s], consumer_threads<KS, KC, kWide>() / 32);
     }
     fence_barrier_init();
   }
@@ -630,7 +675,7 @@ __global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<K
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
 
-  if (warp == consumer_threads<KS, KC>() / 32) {
+  if (warp == consumer_threads<KS, KC, kWide>() / 32) {
     // ---------------- producer warp ----------------
     if (lane == 0) {
       uint32_t it = 0;
@@ -642,12 +687,12 @@ __global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<K
         const int f = fcur = next_frame(prefix, nframes, tile, fcur);
         const hsi_frame& F = frame_at(prm, f);
         const int64_t P = static_cast<int64_t>(F.height) * F.width;
-        const int64_t p0 = static_cast<int64_t>(tile - prefix[f]) * kTile;
-        const int npx = static_cast<int>(P - p0 < kTile ? P - p0 : kTile);
+        const int64_t p0 = static_cast<int64_t>(tile - prefix[f]) * kTilePx;
+        const int npx = static_cast<int>(P - p0 < kTilePx ? P - p0 : kTilePx);
         const uint32_t bytes = static_cast<uint32_t>(((npx + 7) & ~7) * sizeof(T));
         const T* cube = static_cast<const T*>(F.cube);
-        for (int b0 = 0; b0 < F.bands; b0 += CubeTraits<T>::kStageBands) {
-          const int nb = F.bands - b0 < CubeTraits<T>::kStageBands ? F.bands - b0 : CubeTraits<T>::kStageBands;
+        for (int b0 = 0; b0 < F.bands; b0 += kStageBands) {
+          const int nb = F.bands - b0 < kStageBands ? F.bands - b0 : kStageBands;
           const int slot = static_cast<int>(it % kStages);
           const uint32_t round = it / kStages;
           if (*abort_flag || !mbar_wait(&empty[slot], (round & 1u) ^ 1u)) {
@@ -659,7 +704,7 @@ __global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<K
           T* dst = reinterpret_cast<T*>(smem + slot * L.stage_bytes);
           mbar_arrive_expect_tx(&full[slot], bytes * nb);
           for (int i = 0; i < nb; ++i)
-            bulk_g2s(dst + i * kTile, cube + static_cast<int64_t>(b0 + i) * F.plane_stride + p0, bytes,
+            bulk_g2s(dst + i * kTilePx, cube + static_cast<int64_t>(b0 + i) * F.plane_stride + p0, bytes,
                      &full[slot]);
           pending |= 1u << slot;
           pending_parity = (pending_parity & ~(1u << slot)) | ((round & 1u) << slot);
@@ -677,7 +722,7 @@ __global__ void __launch_bounds__(consumer_threads<KS, KC>() + 32, fused_banks<K
   if constexpr (fused_banks<KS, KC>()) {
     float* filt = reinterpret_cast<float*>(smem + L.filt_off);
     float* scale = reinterpret_cast<float*>(smem + L.scale_off);
-    consumer_loop_fused<T, KS, KC, kStages>(prm, prefix, total_tiles, smem, L.stage_bytes, full, empty, abort_flag,
+    consumer_loop_fused<T, KS, KC, kStages, kWide>(prm, prefix, total_tiles, smem, L.stage_bytes, full, empty, abort_flag,
                                             filt, scale, threadIdx.x, lane);
     return;
   }
@@ -1200,12 +1245,12 @@ int round_filters(int n) {
   return 16;
 }
 
-template <typename T, int KS, int KC>
-int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaStream_t stream) {
+template <typename T, int KS, int KC, bool kWide>
+int launch_form(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaStream_t stream) {
   constexpr int kGroups = score_groups<KS, KC>();
-  const SmemLayout L = smem_layout<T>(kGroups, max_bands, score_slots<KS, KC>(), score_stages<T, KS, KC>());
-  const int threads = consumer_threads<KS, KC>() + 32;
-  auto kernel = score_kernel<T, KS, KC>;
+  const SmemLayout L = smem_layout<T, kWide>(kGroups, max_bands, score_slots<KS, KC>(), score_stages<T, KS, KC, kWide>());
+  const int threads = consumer_threads<KS, KC, kWide>() + 32;
+  auto kernel = score_kernel<T, KS, KC, kWide>;
   // The layout follows the band count of the call.  The device's limit for
   // this kernel only ever rises, so a concurrent call with fewer bands cannot
   // lower it below this launch's layout; residency is per layout and device.
@@ -1218,6 +1263,31 @@ int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaSt
   const int grid = sm_count() * per;
   kernel<<<grid, threads, L.total, stream>>>(p, max_bands);
   return static_cast<int>(cudaGetLastError());
+}
+
+template <typename T, int KS, int KC>
+int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaStream_t stream) {
+  // Sixteen filters of a pixel keep the FP32 scorer on the banks' shared-memory
+  // reads, which the wide form halves: it takes 0.85 to 0.93 of the narrow
+  // form's time a pixel (four 1024 x 1024 x 113 frames 427 us, 459; 2 x 1024 x
+  // 1024 x 224 384, 441).  Its tiles are larger, so a short launch can leave more
+  // of the SMs' last round empty (640 x 640 x 113: 63 us, 60): it is taken when the
+  // busiest SM's pixels are at most 1.15 times the narrow form's.  Frames in a
+  // device table have unknown sizes here and take the narrow form.
+  if constexpr (sizeof(T) == 4 && fused_banks<KS, KC>() && KS + KC == 16) {
+    int64_t wide = 0, narrow = 0;  // tiles
+    if (!p.table)
+      for (int f = 0; f < p.num_frames; ++f) {
+        const int64_t P = static_cast<int64_t>(p.inline_frames[f].height) * p.inline_frames[f].width;
+        wide += div_up<int64_t>(P, tile_px<true>());
+        narrow += div_up<int64_t>(P, tile_px<false>());
+      }
+    const int64_t sms = sm_count();
+    if (wide > 0 &&
+        100 * div_up(wide, sms) * tile_px<true>() <= 115 * div_up(narrow, sms) * tile_px<false>())
+      return launch_form<T, KS, KC, true>(p, max_bands, ctas_per_sm, stream);
+  }
+  return launch_form<T, KS, KC, false>(p, max_bands, ctas_per_sm, stream);
 }
 
 template <typename T, int KS>

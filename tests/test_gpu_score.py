@@ -326,6 +326,44 @@ def test_batched_frames_inline_and_device_table(hsi, orc):
         _check_sam(orc, host, targets, best.cpu().numpy(), bt.cpu().numpy(), maps.cpu().numpy())
 
 
+@pytest.mark.parametrize("ks,kc", [(8, 8), (16, 0), (0, 16), (13, 0), (5, 7)])
+@pytest.mark.parametrize("shapes,B", [([(300, 300)], 113), ([(300, 300)], 1), ([(521, 695)], 8), ([(521, 695)], 9),
+                                      ([(1, 132609)], 224), ([(300, 301), (7, 5), (299, 300)], 31)])
+def test_wide_form_equals_narrow_form(hsi, shapes, B, ks, kc):
+    """Sixteen filter slots over tiles of 896 pixels (host descriptors) and of 512 (a
+    device table) run the same sums in the same order: every output bit is equal, at
+    remainders of the stages' 8 bands and of the tiles, with maps on and off 16 bytes."""
+    gen = torch.Generator(device="cuda").manual_seed(7 * B + 100 * ks + kc)
+    out = []
+    frames = ([], [])
+    for n, (H, W) in enumerate(shapes):
+        P = H * W
+        stride = (P + 7) // 8 * 8
+        cube = torch.rand((B, stride), generator=gen, device="cuda")
+        sam = torch.rand((max(ks, 1), B), generator=gen, device="cuda")
+        cem = torch.randn((max(kc, 1), B), generator=gen, device="cuda")
+        norms = sam.double().square().sum(1).sqrt().float()
+        for form in (0, 1):
+            r = dict(sm=torch.full((max(ks, 1), P + n), -7.0, device="cuda"), sb=torch.full((P,), -7.0, device="cuda"),
+                     st=torch.full((P,), -7, dtype=torch.int32, device="cuda"),
+                     cm=torch.full((max(kc, 1), P + n), -7.0, device="cuda"), cb=torch.full((P,), -7.0, device="cuda"),
+                     ct=torch.full((P,), -7, dtype=torch.int32, device="cuda"))
+            frames[form].append(hsi.make_frame(
+                cube, H, W, B, sam_targets=sam if ks else None, sam_norms=norms if ks else None,
+                cem_weights=cem if kc else None, sam_maps=r["sm"] if ks else None, sam_best=r["sb"] if ks else None,
+                sam_best_target=r["st"] if ks else None, cem_maps=r["cm"] if kc else None,
+                cem_best=r["cb"] if kc else None, cem_best_target=r["ct"] if kc else None, map_stride=P + n))
+            out.append((n, form, r, cube, sam, cem, norms))
+    hsi.score_frames(frames[0])
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    hsi.score_frames_device(hsi.frame_table(frames[1]), len(shapes), max_bands=B, max_sam=ks, max_cem=kc, status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for a, b in zip(out[::2], out[1::2]):
+        for key in a[2]:
+            assert torch.equal(a[2][key], b[2][key]), key
+
+
 def test_device_table_rejects_frames_outside_bounds(hsi):
     """A frame with more bands than the launch allows is skipped, not overrun."""
     H, W, B = 8, 8, 64

@@ -459,9 +459,9 @@ class Workload:
             events[3].record(stream)
         return launches
 
-    # per group of up to 64 frames: subsample init / partial / finalize, GEMM,
-    # range check, rescale, conditional GEMM re-run, reduce, finalize
-    stats_launches = 9
+    # per group of up to 64 frames: subsample, its reduction, GEMM, range check,
+    # rescale, conditional GEMM re-run, reduce, finalize
+    stats_launches = 8
 
 
 def algorithmic_bytes_score(frames, cem, esize=4):

@@ -114,26 +114,32 @@ __device__ __forceinline__ bool suppresses(float o, float s, bool earlier) {
 // rows in one block.
 constexpr int kFew = 6;
 constexpr int kRounds = 3;  // rounds whose neighbours a lane keeps: all of them up to radius 4
+// Window rows in the order 0, 1, -1, 2, -2, ..: the side is 2 r + 1 with r up to
+// the map's larger side, which may take the whole of 32 bits, and a row is up to
+// 2^31 pixels, so its neighbours' offsets take 64.
 struct WarpWindow {
-  int side;              // 2 r + 1
-  int offset[kRounds];   // this lane's neighbours as linear offsets; 0 (the candidate itself) past the window
+  unsigned side;           // 2 r + 1
+  int64_t offset[kRounds];  // this lane's neighbours as linear offsets; 0 (the candidate itself) past the window
   bool earlier[kRounds];
 };
-__device__ __forceinline__ void warp_neighbour(int k, int side, int& dx, int& dy) {
+__device__ __forceinline__ int window_row(unsigned i) {
+  return (i & 1u) ? static_cast<int>(i / 2u) + 1 : -static_cast<int>(i / 2u);
+}
+__device__ __forceinline__ void warp_neighbour(unsigned k, unsigned side, int& dx, int& dy) {
   dx = dy = 0;
-  if (k >= static_cast<int64_t>(side) * side) return;
-  const int i = k / side;  // rows 0, 1, -1, 2, -2, ..
-  dy = (i & 1) ? (i + 1) / 2 : -(i / 2);
-  dx = k - i * side - side / 2;
+  if (k >= static_cast<uint64_t>(side) * side) return;
+  const unsigned i = k / side;
+  dy = window_row(i);
+  dx = static_cast<int>(k - i * side) - static_cast<int>(side / 2u);
 }
 __device__ __forceinline__ WarpWindow warp_window(const Job& J) {
   WarpWindow w;
-  w.side = 2 * J.radius + 1;
+  w.side = 2u * static_cast<unsigned>(J.radius) + 1u;
 #pragma unroll
   for (int k = 0; k < kRounds; ++k) {
     int dx, dy;
     warp_neighbour(32 * k + (threadIdx.x & 31), w.side, dx, dy);
-    w.offset[k] = dy * J.width + dx;
+    w.offset[k] = static_cast<int64_t>(dy) * J.width + dx;
     w.earlier[k] = dy < 0 || (dy == 0 && dx < 0);
   }
   return w;
@@ -141,26 +147,26 @@ __device__ __forceinline__ WarpWindow warp_window(const Job& J) {
 template <int R, bool HIGHER>
 __device__ __forceinline__ bool warp_suppressed(const Job& J, const WarpWindow& w, int x, int y, float s) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int r = R <= kLaneR ? R : w.side / 2;
+  const int r = R <= kLaneR ? R : static_cast<int>(w.side / 2u);
   constexpr int kHeld = R <= 2 ? 1 : R == 3 ? 2 : kRounds;
   const float* p = J.score + static_cast<int64_t>(y) * J.width + x;
-  int i = 0;  // first row still to look at
+  unsigned i = 0;  // first row still to look at
   if (x >= r && x < J.width - r && y >= r && y < J.height - r) {
     // the whole window lies in the map; the candidate itself never suppresses
 #pragma unroll
     for (int k = 0; k < kHeld; ++k) {
-      if (k > 0 && 32 * k >= static_cast<int64_t>(w.side) * w.side) return false;
+      if (k > 0 && 32u * k >= static_cast<uint64_t>(w.side) * w.side) return false;
       if (__any_sync(kAll, suppresses<HIGHER>(__ldg(p + w.offset[k]), s, w.earlier[k]))) return true;
     }
     if (R <= kLaneR) return false;
     i = 32 * kHeld / w.side;
   }
   // windows across the map's edge, and what is left of larger ones: row by row
-  const int lo = max(x - r, 0), hi = min(x + r, J.width - 1);
+  const int lo = max(x - r, 0), hi = r < J.width - 1 - x ? x + r : J.width - 1;
 #pragma unroll 1
   for (; i < w.side; ++i) {
-    const int dy = (i & 1) ? (i + 1) / 2 : -(i / 2);
-    if (static_cast<unsigned>(y + dy) >= static_cast<unsigned>(J.height)) continue;
+    const int dy = window_row(i);
+    if (static_cast<unsigned>(y) + static_cast<unsigned>(dy) >= static_cast<unsigned>(J.height)) continue;
     const float* row = p + static_cast<int64_t>(dy) * J.width - x;
     for (int n0 = lo; n0 <= hi; n0 += 32) {
       const int nx = n0 + (threadIdx.x & 31);

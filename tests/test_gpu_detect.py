@@ -221,3 +221,29 @@ def test_candidate_densities_bit_exact(hsi, orc, shape, radius, share):
     n, got = _gpu_detect(hsi, score, None, H, W, share, radius, False)
     assert n == n0
     assert _tuples(got) == _tuples(want)
+
+
+@pytest.mark.parametrize("width, radius", [(1 << 29, 4), (1 << 30, 2)])
+def test_rows_whose_window_spans_more_than_2_31_pixels(hsi, width, radius):
+    """A window's rows lie radius * width pixels apart, past 32 bits for the widest maps the
+    segment limit admits."""
+    H = 2 * radius + 1
+    need = 5 * width * H
+    if torch.cuda.mem_get_info()[0] < need + (4 << 30):
+        pytest.skip("needs a GPU with 28 GB free")
+    score = torch.full((H, width), -1.0, device="cuda")
+    y = radius
+    beaten = [(5000, -radius, -1), (70001, radius, radius), (width // 2, -radius, radius), (width - 9000, radius, -radius)]
+    for x, dy, dx in beaten:  # a better neighbour at the far edge of the window
+        score[y, x] = 1.0
+        score[y + dy, x + dx] = 2.0
+    alone = [20000, width // 2 + 777, width - 3000]
+    for x in alone:
+        score[y, x] = 1.0
+    want = sorted([(y, x) for x in alone] + [(y + dy, x + dx) for x, dy, dx in beaten])
+    count, out = hsi.detect(score, None, H, width, 0.5, radius, hsi.HIGHER_IS_BETTER, 64)
+    torch.cuda.synchronize()
+    n, got = hsi.detections_to_numpy(count, out, 64)
+    del score
+    torch.cuda.empty_cache()
+    assert [(int(d["y"]), int(d["x"])) for d in got] == want and n == len(want)

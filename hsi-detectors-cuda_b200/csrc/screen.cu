@@ -22,6 +22,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <type_traits>
 
 #include "synth.h"
@@ -502,8 +503,15 @@ cudaError_t launch_train(const float* params, int B, const float* X, const float
   return cudaGetLastError();
 }
 
-size_t train_bytes(int B, int n) {
-  return sizeof(float) * static_cast<size_t>(train_ctas(n)) * static_cast<size_t>(partial_stride(B)) + 256;
+// Room for the partials of any batch of up to n samples at any band count, as the
+// callers' workspace had before: batches of 32-sample chunks (up to 4736 samples)
+// leave up to 148 partials, 8192 samples in 64-sample chunks 128, so that the
+// latter's own would be too small for a shorter batch.
+size_t train_bytes(int n) {
+  const int chunks = n / 32 + (n % 32 != 0);
+  return sizeof(float) * static_cast<size_t>(std::min(chunks, kTrainMaxCtas)) *
+             static_cast<size_t>(partial_stride(HSI_MAX_BANDS)) +
+         256;
 }
 
 __global__ void adam_kernel(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
@@ -896,7 +904,7 @@ extern "C" HSI_API int hsi_screen_gather(const void* d_cube, int dtype, int64_t 
 
 extern "C" HSI_API size_t hsi_screen_train_workspace_bytes(int bands, int n) {
   if (bands <= 0 || n <= 0) return 0;
-  return train_bytes(bands, n);
+  return train_bytes(n);
 }
 
 extern "C" HSI_API int hsi_screen_gradients(const float* d_params, int bands, const float* d_features,
@@ -905,7 +913,7 @@ extern "C" HSI_API int hsi_screen_gradients(const float* d_params, int bands, co
                                             hsi_stream_t stream) {
   if (!d_params || !d_features || !d_labels || !d_grads || n <= 0 || bands <= 0 || bands > HSI_MAX_BANDS)
     return HSI_E_INVALID;
-  if (!d_workspace || workspace_bytes < train_bytes(bands, n)) return HSI_E_WORKSPACE;
+  if (!d_workspace || workspace_bytes < train_bytes(n)) return HSI_E_WORKSPACE;
   const cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   float* partials = static_cast<float*>(d_workspace);
   // 16-byte feature copies need every row on 16 bytes

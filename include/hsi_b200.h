@@ -362,7 +362,9 @@ HSI_API int hsi_screen_gather(const void* d_cube, int dtype, int64_t plane_strid
                               const int32_t* d_index, int n, float* d_features, hsi_stream_t stream);
 /* Mean weighted binary cross-entropy on the logit (positives weighted by
  * pos_weight) and its gradient for every parameter (d_grads, param-count
- * floats); `d_loss` (nullable) receives the loss. */
+ * floats); `d_loss` (nullable) receives the loss.  A workspace of
+ * hsi_screen_train_workspace_bytes(bands, n) serves every batch of up to n
+ * samples, at any band count. */
 HSI_API size_t hsi_screen_train_workspace_bytes(int bands, int n);
 HSI_API int hsi_screen_gradients(const float* d_params, int bands, const float* d_features, const float* d_labels,
                                  int n, float pos_weight, float* d_grads, float* d_loss, void* d_workspace,

@@ -256,3 +256,16 @@ def test_conversions_and_gather_reject_bad_arguments_on_the_host():
     assert L.hsi_gather_candidates(fake, hsi.F16, 4096, 113, 64, None, fake, 100, fake, 100, None) == hsi.E_INVALID
     assert L.hsi_gather_candidates(fake, hsi.F16, 4096, 113, 64, fake, fake, 100, fake, 99, None) == hsi.E_INVALID
     assert L.hsi_gather_candidates(fake, 4, 4096, 113, 64, fake, fake, 100, fake, 100, None) == hsi.E_INVALID
+
+
+def test_training_workspace_serves_shorter_batches():
+    """The screen's training workspace grows with the batch and does not depend on the
+    bands, so that one sized at a program's largest batch serves every shorter one."""
+    import hsi_b200 as hsi
+    size = hsi.lib().hsi_screen_train_workspace_bytes
+    assert size(0, 32) == size(113, 0) == size(113, -1) == 0
+    batches = [1, 31, 32, 33, 64, 1000, 3500, 4700, 4735, 4736, 4737, 4800, 6000, 8192, 9472, 9473, 1 << 20, 2**31 - 1]
+    for bands in (1, 16, 64, 65, 113, 224, 256):
+        sizes = [size(bands, n) for n in batches]
+        assert sizes[0] > 0 and sizes == sorted(sizes)
+        assert sizes == [size(1, n) for n in batches]

@@ -112,6 +112,26 @@ def test_gradients_over_sample_chunks(hsi, orc, B, n, off):
         pos += size
 
 
+@pytest.mark.parametrize("B,sized,n", [((224, 224), 8192, 4700), ((113, 113), 6000, 3500), ((16, 256), 8192, 4736)])
+def test_gradients_in_the_workspace_of_a_larger_batch(hsi, B, sized, n):
+    """The workspace of a program's largest batch serves a shorter one (and more bands),
+    with the gradients of a workspace of its own."""
+    L = hsi.lib()
+    p, Bp = _params(hsi, B[1], 7)
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    X = torch.zeros((Bp, n), device="cuda")
+    X[:B[1]] = torch.randn((B[1], n), generator=gen, device="cuda").bfloat16().float()
+    y = (torch.rand(n, generator=gen, device="cuda") < 0.2).float()
+    grads = []
+    for wb in (L.hsi_screen_train_workspace_bytes(B[0], sized), L.hsi_screen_train_workspace_bytes(B[1], n)):
+        ws = torch.empty(wb, dtype=torch.uint8, device="cuda")
+        grads.append(torch.full_like(p, np.nan))
+        assert L.hsi_screen_gradients(_p(p), B[1], _p(X), _p(y), n, C.c_float(3.0), _p(grads[-1]), None, _p(ws), wb,
+                                      None) == 0
+    torch.cuda.synchronize()
+    assert torch.equal(grads[0], grads[1])
+
+
 def test_adam_step_moves_against_the_gradient(hsi):
     L = hsi.lib()
     B = 16

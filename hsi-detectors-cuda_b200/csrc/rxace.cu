@@ -38,6 +38,7 @@
 // a barrier per chunk, warps idling above the diagonal).
 #include "common.cuh"
 #include "launch_state.h"
+#include "rxace_panels.h"
 
 #include <algorithm>
 
@@ -46,23 +47,8 @@ namespace {
 
 constexpr int kPxTile = 64;     // pixels per tile
 constexpr int kThreads = 256;
-constexpr int kGroupRows = 8;   // output rows (bands + targets) per group
-constexpr int kChains = 16;     // partial sums of RX per pixel: groups G, G + 16, G + 32 each
-constexpr int kMaxGroups = (HSI_MAX_BANDS + HSI_MAX_FILTERS_PER_PASS) / kGroupRows;
-constexpr int kMaxPairs = (kMaxGroups + 1) / 2;
-constexpr int kWarps = kThreads / 32;
-
-// Where the groups' weights lie (floats from the panels' start, [k][8 rows] of
-// `bands[g]` bands) and which warp takes which pairs of groups (2 i, 2 i + 1).
-struct Panels {
-  int groups;
-  int kpad;                       // bands rounded up to 8
-  int floats;                     // of all panels
-  int offset[kMaxGroups];
-  short bands[kMaxGroups];
-  unsigned char first[kWarps + 1];  // warp w's pairs: pair[first[w]] .. pair[first[w + 1] - 1], ascending
-  unsigned char pair[kMaxPairs];
-};
+constexpr int kWarps = kSimtWarps;
+static_assert(kThreads == 32 * kWarps, "a list of pairs per warp");
 
 // Prepared operands in the workspace (FP32 path).
 struct SimtOperands {
@@ -71,41 +57,6 @@ struct SimtOperands {
   float* mean_lo;
   float* uu;       // [T]
 };
-
-__host__ __device__ inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
-
-Panels make_panels(int B, int T) {
-  Panels p{};
-  p.groups = (B + T + kGroupRows - 1) / kGroupRows;
-  p.kpad = round_up(B, kGroupRows);
-  const int pairs = (p.groups + 1) / 2;
-  for (int g = 0; g < p.groups; ++g)  // rows above B end their dot product at the diagonal; target rows are dense
-    p.bands[g] = static_cast<short>(std::min((g + 1) * kGroupRows, p.kpad));
-  // longest pair first, each to the warp with the least to do
-  int load[kWarps] = {}, warp_of[kMaxPairs];
-  for (int i = pairs - 1; i >= 0; --i) {
-    const int w = static_cast<int>(std::min_element(load, load + kWarps) - load);
-    warp_of[i] = w;
-    load[w] += p.bands[std::min(2 * i + 1, p.groups - 1)];
-  }
-  int n = 0;
-  for (int w = 0; w < kWarps; ++w) {
-    p.first[w] = static_cast<unsigned char>(n);
-    for (int i = 0; i < pairs; ++i)
-      if (warp_of[i] == w) p.pair[n++] = static_cast<unsigned char>(i);
-  }
-  p.first[kWarps] = static_cast<unsigned char>(n);
-  // the two halves of a warp read their weights at the same band: the odd
-  // groups' panels start 64 bytes off, on other banks
-  for (int half = 0; half < 2; ++half) {
-    if (half) p.floats += 16;
-    for (int g = half; g < p.groups; g += 2) {
-      p.offset[g] = p.floats;
-      p.floats += p.bands[g] * kGroupRows;
-    }
-  }
-  return p;
-}
 
 // One thread per weight: rows < B copy W, rows B + t hold v_t = W^T u_t in
 // FP64; the rest are zero.  blockIdx.x: the group, blockIdx.y: 256 weights of
@@ -187,7 +138,8 @@ struct SimtSmem {
   float rx[kChains][kPxTile];
   float zu[HSI_MAX_FILTERS_PER_PASS][kPxTile];
   int done[kMaxPairs + 1];  // tiles whose squares pair i has added (per block, in order)
-  int pad[2];               // y starts on 16 bytes
+  int gave_up;              // a wait ran out: sums are missing
+  int pad;                  // y starts on 16 bytes
   // then y[kpad][kPxTile], the panels, 8 floats that the last band's prefetch reads
 };
 
@@ -214,6 +166,7 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
   for (int b = tid; b < B; b += kThreads) sm.mean[b] = make_float2(op.mean_hi[b], op.mean_lo[b]);
   if (tid < Tn) sm.uu[tid] = op.uu[tid];
   if (tid <= kMaxPairs) sm.done[tid] = 0;
+  if (tid == 0) sm.gave_up = 0;
 
   // this thread's share of a tile: V pixels from px0 on of bands b0, b0 + step, ..
   constexpr int kStep = kThreads / kRowVecs;
@@ -315,10 +268,13 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
       float* sum = &sm.rx[g % kChains][px];
       if (pair >= kChains / 2) {
         // the chain's earlier groups; the wait ends: their warp has them ahead
-        // of anything that waits, and the lowest pair in work waits for none
+        // of anything that waits, and the lowest pair in work waits for none.
+        // Should it run out all the same, the block ends with this tile and its
+        // scores become NaN (there is no status word to set).
         volatile const int* before = &sm.done[pair - kChains / 2];
-        for (uint32_t n = 0; *before < turn && n < kWaitLimit; ++n) {
-        }
+        uint32_t n = 0;
+        while (*before < turn && n < kWaitLimit) ++n;
+        if (n == kWaitLimit) sm.gave_up = 1;
         __threadfence_block();
         part = *reinterpret_cast<const float4*>(sum);
       }
@@ -391,6 +347,18 @@ __global__ void __launch_bounds__(kThreads, BANDS <= 128 ? 2 : 1)
       }
     }
     __syncthreads();  // the next tile's pixels are in, this one's sums read
+    if (sm.gave_up) break;
+  }
+  if (sm.gave_up) {
+    const float nan = __int_as_float(0x7fc00000);
+    for (tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      const int64_t p = tile * kPxTile + tid;
+      if (tid >= kPxTile || p >= pixels) continue;
+      if (out.rx) out.rx[p] = nan;
+      if (out.ace_best) out.ace_best[p] = nan;
+      if (out.ace_target) out.ace_target[p] = -1;
+      for (int t = 0; out.ace_maps && t < Tn; ++t) out.ace_maps[static_cast<int64_t>(t) * out.map_stride + p] = nan;
+    }
   }
 }
 

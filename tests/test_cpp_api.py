@@ -56,6 +56,14 @@ def test_host_only_program_passes_without_a_device():
     assert r.stdout.strip().splitlines()[-1] == "ok host_api", r.stdout
 
 
+def test_plain_rx_ace_schedule_ends_for_every_band_and_target_count():
+    """Host code of the scorer alone: no wait between its warps can last for ever."""
+    _make_tests()
+    r = subprocess.run([os.path.join(BIN, "test_rxace_panels")], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0, r.stdout + r.stderr
+    assert r.stdout.strip().splitlines()[-1] == "ok rxace_panels", r.stdout
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("program", PROGRAMS)
 def test_cpp_program_passes_on_the_device(program):

@@ -154,6 +154,18 @@ def cpu_reference(workload, sample_rows, repeats, threads=None):
     return times, threads, P
 
 
+def cpu_baseline(workload, note=""):
+    """The line's "cpu_baseline": the reference's CPU path on sample frames, or why its
+    library (compiled from its sources by oracle/Makefile) is not there."""
+    try:
+        times, threads, P = cpu_reference(workload, 128, 2)
+    except OSError as e:
+        return {"unavailable": f"{type(e).__name__}: {e}"}
+    t = float(np.mean(times))
+    return {"value": round(threads * P / t / 1e6, 3), "unit": "Mpix/s", "cores": threads, "kind": "reference",
+            "sample": f"{threads} frames of {W}x128x{B}, one per thread{note}, mean of 2 runs"}
+
+
 # Shapes of the same-box GPU comparison of SAM scorers: the plain-SAM
 # configuration (one target) and the SAM+CEM video frame (eight targets).
 SAM_SHAPES = [(520, 696, 113, 1), (1024, 1024, 113, 8)]
@@ -600,10 +612,7 @@ def run_ours(args, workload):
 
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
-        times, threads, P = cpu_reference(workload, 128, 2)
-        t = float(np.mean(times))
-        cpu = {"value": round(threads * P / t / 1e6, 3), "unit": "Mpix/s", "cores": threads, "kind": "reference",
-               "sample": f"{threads} frames of {W}x128x{B}, one per thread, mean of 2 runs"}
+        cpu = cpu_baseline(workload)
 
     if rank == 0:
         line = {
@@ -1044,11 +1053,7 @@ def measure_rxace(args, dist, world, rank, device):
     torch.cuda.empty_cache()
     cpu = None
     if rank == 0 and world == 1 and not args.no_cpu:
-        times, threads, Ps = cpu_reference("rx_ace", 128, 2)
-        t = float(np.mean(times))
-        cpu = {"value": round(threads * Ps / t / 1e6, 3), "unit": "Mpix/s", "cores": threads, "kind": "reference",
-               "sample": f"{threads} frames of {W}x128x{B}, one per thread (moments + statistics + ace_best_cpu "
-                         "with RX), mean of 2 runs"}
+        cpu = cpu_baseline("rx_ace", " (moments + statistics + ace_best_cpu with RX)")
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(REPO, "MEASURED_PEAKS.json")))

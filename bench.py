@@ -451,7 +451,7 @@ class Workload:
         if self.cem:
             hsi.check(L.hsi_scene_moments_batch(self.moment_jobs, self.n, C.c_void_p(self.stats_ws.data_ptr()),
                                                 self.stats_bytes, s), "hsi_scene_moments_batch")
-            launches += self.stats_launches * ((self.n + 63) // 64)
+            launches += moments_launches([(H * W, B)] * self.n)
             # one launch factors every frame (one CTA per frame, FP64)
             hsi.check(L.hsi_build_statistics(self.n, B, TARGETS, LOADING, C.c_void_p(self.moments.data_ptr()),
                                              C.c_void_p(self.targets.data_ptr()), 0, None, None,
@@ -466,14 +466,51 @@ class Workload:
             events[1].record(stream)
         self.counts.zero_()
         hsi.detect_batch(self.jobs, self.det_ws, stream=stream)
-        launches += 2
+        launches += detect_launches(len(self.jobs))
         if events is not None and len(events) > 3:
             events[3].record(stream)
         return launches
 
-    # per group of up to 64 frames: subsample, its reduction, GEMM, range check,
-    # rescale, conditional GEMM re-run, reduce, finalize
-    stats_launches = 8
+
+# ---------------------------------------------------------------------------
+# Kernel launches of the library's calls (the lines' "gpu_launches"; copies and
+# fills are not counted)
+# ---------------------------------------------------------------------------
+
+def moments_launches(frames):
+    """hsi_scene_moments(_batch) over FP32 or FP16 frames of one element type, (pixels, bands) each."""
+    tensor = sum(1 for p, b in frames if p >= 32768 and b <= 127)
+    # groups of up to 64 tensor-path frames: subsample, its reduction, GEMM, range
+    # check, rescale, conditional GEMM re-run, reduce, finalize
+    n = 8 * ((tensor + 63) // 64)
+    for p, b in frames:
+        if p >= 32768 and 127 < b <= 252:
+            n += 9  # the same over six views, and their assembly
+        elif p >= 32768 and 252 < b <= 254:
+            n += 10  # the same over two views, the cross product and the assembly
+        elif p < 32768 or b > 254:
+            n += 6  # plain: three for the reference point, product, reduce, finalize
+    return n
+
+
+def rx_ace_launches(bands, targets, tensor_cores):
+    """Preparation and scorer per pass over the targets."""
+    return 2 * (max(1, -(-targets // min(16, 128 - bands))) if tensor_cores else 1)
+
+
+def detect_launches(maps=1):
+    """Two per 64 maps (of up to 16384 row segments each)."""
+    return 2 * ((maps + 63) // 64)
+
+
+def batch_launches(specs):
+    """One run of the batch runner over (height, width, bands, targets, mosaic) FP32 frames,
+    RX/ACE on the tensor cores up to 127 bands: one scorer launch, the moments, a
+    factorisation and RX/ACE per frame, demosaics, three lists per frame."""
+    n = 1 + moments_launches([(h * w, b) for h, w, b, _, _ in specs]) + detect_launches(3 * len(specs))
+    for _, _, b, t, mosaic in specs:
+        n += (1 if mosaic else 0) + 1 + rx_ace_launches(b, t, b <= 127)
+    return n
 
 
 def algorithmic_bytes_score(frames, cem, esize=4):
@@ -852,13 +889,13 @@ def run_e2e(hsi, torch, wl, stream, args, world):
                                                  C.c_void_p(wl.targets.data_ptr()), 0, None, None,
                                                  C.c_void_p(wl.cem_w[i].data_ptr()),
                                                  C.c_void_p(wl.status[i:i + 1].data_ptr()), None, 0, s), "stats")
-                launches += wl.stats_launches + 1
+                launches += moments_launches([(H * W, B)]) + 1
             hsi.score_frames([frames[i]], stream=stream)
             freed[i].record(stream)
             wl.counts[f:f + 1].zero_()
             hsi.detect(wl.sam_best[i], wl.sam_bt[i], H, W, THRESHOLD, NMS_RADIUS, hsi.LOWER_IS_BETTER, CAPACITY,
                        out=wl.dets[f], count=wl.counts[f:f + 1], workspace=wl.ws[f], stream=stream)
-            launches += 4
+            launches += 1 + detect_launches()
         out_host.copy_(wl.dets, non_blocking=True)
         count_host.copy_(wl.counts, non_blocking=True)
         return launches
@@ -1079,7 +1116,8 @@ def measure_rxace(args, dist, world, rank, device):
                            "tensor_core_speedup": round(plain_kern / kern_ms, 2),
                            "step_speedup": round(plain_ms / ms, 2)},
             "errors_vs_fp64": errors,
-            "cpu_baseline": cpu, "e2e": e2e, "gpu_launches": 6 + 1 + 2, "clocks": clocks.summary(),
+            "cpu_baseline": cpu, "e2e": e2e,
+            "gpu_launches": args.steps * (moments_launches([(P, B)]) + 1 + rx_ace_launches(B, T, True)), "clocks": clocks.summary(),
         }
     del rx, ab, at, maps, sws, tws, pws
     torch.cuda.empty_cache()
@@ -1233,7 +1271,8 @@ def measure_screen(args, dist, world, rank, device):
                                vp(dets), vp(dcount), vp(dws), dws.numel(), s), "final list")
         if ev:
             ev[2].record(stream)
-        return 9 + 6
+        # moments, factorisation, normaliser, screen (pack + inference), proposals, gather, re-scoring, final list
+        return moments_launches([(P, Bs)]) + 1 + 1 + 2 + detect_launches() + 1 + 2 + detect_launches()
 
     def plain_step(src, ev=None):
         if ev:
@@ -1245,7 +1284,7 @@ def measure_screen(args, dist, world, rank, device):
                                     vp(pws), pws_b, s), "plain ace")
         if ev:
             ev[2].record(stream)
-        return 8
+        return moments_launches([(P, Bs)]) + 1 + 2
 
     def timed(fn, steps, warmup):
         """(ms per step, ms per step after the shared statistics, launches)"""
@@ -1437,12 +1476,7 @@ def run_batch(args):
     eager_ms = timed(batch.run, max(2, args.steps // 2))
     ms, eager_ms = max_over_ranks(dist, [ms, eager_ms], device)
     tuning = batch.tuning()
-    # launches per run: demosaic, moments (6 tensor-core / 3 plain), factor, RX/ACE (prep + main per pass),
-    # one scorer launch, the counts memset, two detection launches per 64 lists
-    launches = 1 + 2 * ((3 * BATCH_FRAMES + 63) // 64)
-    for (h, w, b, t, mosaic) in specs:
-        launches += (1 if mosaic else 0) + (6 if (b <= 127 and h * w >= 32768) else 3) + 1
-        launches += 2 * (1 if b > 127 else -(-t // max(1, min(16, 128 - b))))
+    launches = args.steps * batch_launches(specs)
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(REPO, "MEASURED_PEAKS.json")))

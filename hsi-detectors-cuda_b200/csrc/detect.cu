@@ -5,14 +5,16 @@
 // run to run:
 //   1. flags:  one warp per 2048-pixel row segment writes every pixel's
 //              pass/fail as ballot words (a bitmask in the workspace) and the
-//              segment's count.  The map streams through once; only a
+//              segment's count.  The map streams through once; a
 //              candidate (a score past the threshold) looks at its
 //              (2r+1)^2 window, straight from global memory, where the
 //              block's eight warps -- neighbouring rows -- have brought it
-//              into L1.  A neighbour suppresses when it comes first in the
-//              window's order (better score, or the same score at a lower
-//              linear index); out-of-frame neighbours are skipped and NaN
-//              never wins or ties, exactly like the CPU loop.
+//              into L1, and a chunk of 128 pixels with more than a few
+//              candidates at the windows of all of them together.  A
+//              neighbour suppresses when it comes first in the window's order
+//              (better score, or the same score at a lower linear index);
+//              out-of-frame neighbours are skipped and NaN never wins or
+//              ties, exactly like the CPU loop.
 //   2. emit:   a block takes eight segments of one map, adds up the counts of
 //              the segments before them, and each warp writes its segment's
 //              detections at offset + in-segment rank, dropping (but having
@@ -40,8 +42,9 @@ constexpr int kSeg = 2048;                   // pixels per row segment
 constexpr int kWordsPerSeg = kSeg / 32;      // 64
 constexpr int kMaxJobs = 64;
 constexpr int kChunk = 128;                  // pixels a warp takes at a time, four per lane
-constexpr int kLaneR = 4;                    // largest radius of the lanes' own windows (one float4 group each side)
-constexpr int kFilterR = 2;                  // their radius ahead of a larger one
+constexpr int kGroupR = 2;                   // largest radius of the lanes' own windows on 16-byte groups
+constexpr int kHeldR = 4;                    // largest radius with an instance of its own
+constexpr int kDenseR = 8;                   // largest radius of a whole chunk's windows
 // A block of emit reads the counts of all earlier segments of its map: 2 KB on
 // average for 1024 rows.  At 16384 segments (a 16384-row map) the 2048 blocks
 // read 64 MB of L2 together, about what a scan launch costs; the sums grow
@@ -102,25 +105,25 @@ __device__ __forceinline__ bool suppresses(float o, float s, bool earlier) {
 // One candidate by a whole warp, a lane per neighbour and round, rows nearest
 // the candidate first (smooth maps decide in the first round): any radius.
 // A few per cent of the pixels are candidates, so a 128-pixel chunk has two or
-// three; they cost about 20 instructions each here, where the lanes' own
-// windows (below) cost 200 to 500 for the chunk however few of its pixels are
-// candidates.  So up to kFew candidates of a chunk go one by one; more take
-// the lanes' windows, of the whole radius up to kLaneR and of kFilterR above
-// it, which leave the warp a twenty-fifth of the pixels or so.
-// 64 maps of 1024 x 1024 with 0.05, 1, 5 and 30 % of uniform random scores
-// past the threshold, radius 2: 126, 209, 375 and 394 us for both launches;
-// the ring-buffer tiles before (one barrier per row, then a scan launch) took
-// 415 to 455.  One 64 x 96 map: 5.4 us against 69, where a tile walked its 64
-// rows in one block.
-constexpr int kFew = 6;
-constexpr int kRounds = 3;  // rounds whose neighbours a lane keeps: all of them up to radius 4
+// three; they cost about 20 instructions each here, where the whole chunk's
+// windows (below) cost some hundreds however few of its pixels are candidates.
+// So up to kFew candidates of a chunk go one by one.  Eight 1024 x 1024 maps
+// with 5 % of uniform random scores past the threshold (6.4 a chunk), kFew 3, 6
+// and 10: radius 1 42, 50 and 59 us, 2 58, 55 and 60, 4 74, 80 and 85, 8 99, 109
+// and 123, 12 156, 149 and 147.
+// 64 such maps with 1 and 30 % past the threshold, radius 2: 206 and 409 us for
+// both launches; the ring-buffer tiles before (one barrier per row, then a scan
+// launch) took 444 and 478.  One 64 x 96 map: 5.4 us against 69, where a tile
+// walked its 64 rows in one block.
+constexpr int kFew = 4;
+constexpr int kRounds = 3;       // rounds whose neighbours a lane keeps: all of them up to radius kHeldR
+constexpr unsigned kFlatR = 16;  // largest radius whose further rounds run across the window's rows
 // Window rows in the order 0, 1, -1, 2, -2, ..: the side is 2 r + 1 with r up to
 // the map's larger side, which may take the whole of 32 bits, and a row is up to
 // 2^31 pixels, so its neighbours' offsets take 64.
 struct WarpWindow {
-  unsigned side;           // 2 r + 1
-  int64_t offset[kRounds];  // this lane's neighbours as linear offsets; 0 (the candidate itself) past the window
-  bool earlier[kRounds];
+  unsigned side;               // 2 r + 1
+  int dx[kRounds], dy[kRounds];  // this lane's neighbours; (0, 0), the candidate itself, past the window
 };
 __device__ __forceinline__ int window_row(unsigned i) {
   return (i & 1u) ? static_cast<int>(i / 2u) + 1 : -static_cast<int>(i / 2u);
@@ -136,40 +139,46 @@ __device__ __forceinline__ WarpWindow warp_window(const Job& J) {
   WarpWindow w;
   w.side = 2u * static_cast<unsigned>(J.radius) + 1u;
 #pragma unroll
-  for (int k = 0; k < kRounds; ++k) {
-    int dx, dy;
-    warp_neighbour(32 * k + (threadIdx.x & 31), w.side, dx, dy);
-    w.offset[k] = static_cast<int64_t>(dy) * J.width + dx;
-    w.earlier[k] = dy < 0 || (dy == 0 && dx < 0);
-  }
+  for (int k = 0; k < kRounds; ++k) warp_neighbour(32 * k + (threadIdx.x & 31), w.side, w.dx[k], w.dy[k]);
   return w;
+}
+// Whether the neighbour at (x + dx, y + dy), if the map has it, suppresses the candidate s at (x, y).
+template <bool HIGHER>
+__device__ __forceinline__ bool neighbour_suppresses(const Job& J, int x, int y, int dx, int dy, float s) {
+  const int nx = x + dx, ny = y + dy;
+  const bool in = static_cast<unsigned>(nx) < static_cast<unsigned>(J.width) &&
+                  static_cast<unsigned>(ny) < static_cast<unsigned>(J.height);
+  const float o = in ? __ldg(J.score + static_cast<int64_t>(ny) * J.width + nx) : __int_as_float(0x7fc00000);
+  return suppresses<HIGHER>(o, s, dy < 0 || (dy == 0 && dx < 0));
 }
 template <int R, bool HIGHER>
 __device__ __forceinline__ bool warp_suppressed(const Job& J, const WarpWindow& w, int x, int y, float s) {
   constexpr unsigned kAll = 0xffffffffu;
-  const int r = R <= kLaneR ? R : static_cast<int>(w.side / 2u);
   constexpr int kHeld = R <= 2 ? 1 : R == 3 ? 2 : kRounds;
-  const float* p = J.score + static_cast<int64_t>(y) * J.width + x;
-  unsigned i = 0;  // first row still to look at
-  if (x >= r && x < J.width - r && y >= r && y < J.height - r) {
-    // the whole window lies in the map; the candidate itself never suppresses
 #pragma unroll
-    for (int k = 0; k < kHeld; ++k) {
-      if (k > 0 && 32u * k >= static_cast<uint64_t>(w.side) * w.side) return false;
-      if (__any_sync(kAll, suppresses<HIGHER>(__ldg(p + w.offset[k]), s, w.earlier[k]))) return true;
+  for (int k = 0; k < kHeld; ++k)
+    if (__any_sync(kAll, neighbour_suppresses<HIGHER>(J, x, y, w.dx[k], w.dy[k], s))) return true;
+  if constexpr (R <= kHeldR) return false;
+  const int lane = threadIdx.x & 31, r = static_cast<int>(w.side / 2u);
+  if (w.side <= 2 * kFlatR + 1 && 2 * (min(y + r, J.height - 1) - max(y - r, 0)) >= r) {
+#pragma unroll 1
+    for (unsigned k = 32 * kHeld; k < w.side * w.side; k += 32) {
+      int dx, dy;
+      warp_neighbour(k + lane, w.side, dx, dy);
+      if (__any_sync(kAll, neighbour_suppresses<HIGHER>(J, x, y, dx, dy, s))) return true;
     }
-    if (R <= kLaneR) return false;
-    i = 32 * kHeld / w.side;
+    return false;
   }
-  // windows across the map's edge, and what is left of larger ones: row by row
+  // rows of more than a warp's lanes, or most of them outside the map: row by row
+  const float* p = J.score + static_cast<int64_t>(y) * J.width + x;
   const int lo = max(x - r, 0), hi = r < J.width - 1 - x ? x + r : J.width - 1;
 #pragma unroll 1
-  for (; i < w.side; ++i) {
+  for (unsigned i = 32 * kHeld / w.side; i < w.side; ++i) {
     const int dy = window_row(i);
     if (static_cast<unsigned>(y) + static_cast<unsigned>(dy) >= static_cast<unsigned>(J.height)) continue;
     const float* row = p + static_cast<int64_t>(dy) * J.width - x;
     for (int n0 = lo; n0 <= hi; n0 += 32) {
-      const int nx = n0 + (threadIdx.x & 31);
+      const int nx = n0 + lane;
       const bool in = nx <= hi;
       const float o = __ldg(in ? row + nx : p);
       if (__any_sync(kAll, suppresses<HIGHER>(o, s, in && (dy < 0 || (dy == 0 && nx < x))))) return true;
@@ -178,22 +187,152 @@ __device__ __forceinline__ bool warp_suppressed(const Job& J, const WarpWindow& 
   return false;
 }
 
-// One lane's candidate s at (x, y) against its whole window of radius R.
-template <int R, bool HIGHER>
-__device__ __forceinline__ bool lane_suppressed(const Job& J, int x, int y, float s) {
-  bool in[2 * R + 1];
+// ---- the windows of a whole chunk --------------------------------------------
+//
+// Slot j of lane l is column 32 j + l of the chunk; slot 4 holds the columns
+// beside it, lanes 16..31 those on its left (slot -1) and lanes 0..15 those on
+// its right.
+struct Columns {
+  float v[5];
+};
+
+template <bool HIGHER>
+__device__ __forceinline__ float first_of(float a, float b) { return HIGHER ? fmaxf(a, b) : fminf(a, b); }  // NaN never
+template <bool HIGHER>
+__device__ __forceinline__ Columns first_of(const Columns& a, const Columns& b) {
+  Columns c;
 #pragma unroll
-  for (int dx = -R; dx <= R; ++dx) in[dx + R] = x + dx >= 0 && x + dx < J.width;
-  bool hit = false;
+  for (int j = 0; j < 5; ++j) c.v[j] = first_of<HIGHER>(a.v[j], b.v[j]);
+  return c;
+}
+// The columns d to the right (d <= 8): every slot.
+__device__ __forceinline__ Columns right_of(const Columns& a, int d) {
+  const int lane = threadIdx.x & 31;
+  const bool wraps = lane < d;  // the taker, d lanes lower around the warp, wants the next slot's
+  Columns c;
 #pragma unroll
-  for (int dy = -R; dy <= R; ++dy) {
-    if (y + dy < 0 || y + dy >= J.height) continue;
-    const float* p = J.score + static_cast<int64_t>(y + dy) * J.width + x;
+  for (int j = 0; j < 5; ++j)
+    c.v[j] = __shfl_sync(0xffffffffu, wraps ? a.v[j == 4 ? 0 : j + 1] : a.v[j], (lane + d) & 31);
+  return c;
+}
+// The columns d to the left (d <= 8): slots 0..3.
+__device__ __forceinline__ Columns left_of(const Columns& a, int d) {
+  const int lane = threadIdx.x & 31;
+  const bool wraps = lane >= 32 - d;
+  Columns c;
 #pragma unroll
-    for (int dx = -R; dx <= R; ++dx)
-      if ((dx != 0 || dy != 0) && in[dx + R]) hit |= suppresses<HIGHER>(__ldg(p + dx), s, dy < 0 || (dy == 0 && dx < 0));
+  for (int j = 0; j < 4; ++j)
+    c.v[j] = __shfl_sync(0xffffffffu, wraps ? a.v[j == 0 ? 4 : j - 1] : a.v[j], (lane - d) & 31);
+  c.v[4] = c.v[3];
+  return c;
+}
+
+// The chunks of a segment with more than kFew candidates (bit i of `chunks`: the
+// columns from xs + 128 i on) at the job's radius, 1 and up: their mask words;
+// returns how many pixels pass.  A neighbour suppresses by its score and by
+// whether it comes before or after the candidate, so the candidate passes when
+// the first score of the rows above and of its row's columns on the left is not
+// as good as its own, and that of the rows below and of the columns on the
+// right is not better.  Each column's first scores above and below are found
+// once, by one coalesced load a row and 32 columns; the window's width is
+// covered by doubling, with shuffles.  The eight neighbours come first: they
+// leave few pixels of a smooth map, which go one by one, and a ninth of a
+// random one.  So do the pixels that pass at kDenseR where the radius is larger.
+// 2 r + 1 loads of five slots and some 250 instructions for the 128 pixels.  Eight
+// random 1024 x 1024 maps, 30 % past the threshold: radius 3 68 us, 4 77, 5 85, 8
+// 103; 1023 x 1021 the same.  A window per pixel (49 and 81 neighbours) took 89
+// and 122 us on 16-byte groups, 180 and 310 on rows that do not start on 16
+// bytes, and the ring-buffer tiles before 111, 127, 262 and 368.
+// One copy behind all instances of flag_segment, which outgrow the instruction
+// cache otherwise; a call from inside their loops spilled their registers.
+template <bool HIGHER>
+__device__ __forceinline__ uint32_t dense_chunks(const Job& J, int y, int xs, unsigned chunks, uint32_t* mask) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31;
+  const float nan = __int_as_float(0x7fc00000);
+  const int width = J.width, height = J.height, r = min(J.radius, kDenseR);
+  const float threshold = J.threshold;
+  uint32_t total = 0;
+#pragma unroll 1
+  for (; chunks != 0u; chunks &= chunks - 1u) {
+    const int xc = xs + kChunk * (__ffs(chunks) - 1);
+    const int left = width - xc - lane;  // columns from this lane's first on
+    const bool beside = lane >= 16 ? (xc > 0 && lane >= 32 - r) : (lane < r && left > 128);
+    const int xb = lane >= 16 ? lane - 32 : 128 + lane;
+    const float* centre = J.score + static_cast<int64_t>(y) * width + xc;
+    const auto load = [&](int dy) {
+      const float* p = centre + static_cast<int64_t>(dy) * width;
+      Columns c;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) c.v[j] = left > 32 * j ? __ldg(p + lane + 32 * j) : nan;
+      c.v[4] = beside ? __ldg(p + xb) : nan;
+      return c;
+    };
+    const Columns none{{nan, nan, nan, nan, nan}};
+    Columns here = load(0), above = y >= 1 ? load(-1) : none, below = height - y > 1 ? load(1) : none;
+    const Columns s = here;
+    uint32_t word[4];  // bit l of word j: column xc + 32 j + l
+    const auto pass = [&](const Columns& before, const Columns& after) {
+      int n = 0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        word[j] = __ballot_sync(kAll, over_threshold<HIGHER>(s.v[j], threshold) &&
+                                          !suppresses<HIGHER>(before.v[j], s.v[j], true) &&
+                                          !suppresses<HIGHER>(after.v[j], s.v[j], false));
+        n += __popc(word[j]);
+      }
+      return n;
+    };
+    const Columns l = first_of<HIGHER>(above, here), rr = first_of<HIGHER>(here, below);
+    int n = pass(first_of<HIGHER>(first_of<HIGHER>(left_of(l, 1), above), right_of(above, 1)),
+                 first_of<HIGHER>(first_of<HIGHER>(right_of(rr, 1), below), left_of(below, 1)));
+    bool decided = J.radius == 1;
+    if (!decided && n > kFew) {
+#pragma unroll 2
+      for (int d = 2; d <= r; ++d) {
+        const Columns a = y >= d ? load(-d) : none, b = height - y > d ? load(d) : none;
+        above = first_of<HIGHER>(above, a);
+        below = first_of<HIGHER>(below, b);
+      }
+      // the first of q columns from each one on, q the largest power of two <= r;
+      // 2 q then covers more than half of the window of 2 r + 1
+      int q = 1;
+#pragma unroll 1
+      for (; 2 * q <= r; q *= 2) {
+        above = first_of<HIGHER>(above, right_of(above, q));
+        below = first_of<HIGHER>(below, right_of(below, q));
+        here = first_of<HIGHER>(here, right_of(here, q));
+      }
+      above = first_of<HIGHER>(above, right_of(above, q));
+      below = first_of<HIGHER>(below, right_of(below, q));
+      const int rest = 2 * q - r - 1;  // the 2 q columns that end the window start here, on the left of the pixel
+      n = pass(first_of<HIGHER>(first_of<HIGHER>(left_of(above, r), left_of(above, rest)),
+                                first_of<HIGHER>(left_of(here, r), left_of(here, q))),
+               first_of<HIGHER>(first_of<HIGHER>(left_of(below, r), left_of(below, rest)),
+                                first_of<HIGHER>(right_of(here, 1), right_of(here, r - q + 1))));
+      decided = J.radius <= kDenseR;
+    }
+    uint32_t m = lane < 2 ? (lane == 0 ? word[0] : word[1]) : (lane == 2 ? word[2] : word[3]);
+    if (!decided && n > 0) {
+      const WarpWindow ww = warp_window(J);
+      uint32_t todo = lane < 4 ? m : 0u;
+      for (unsigned lanes = __ballot_sync(kAll, todo != 0u); lanes != 0u; lanes = __ballot_sync(kAll, todo != 0u)) {
+        const int j = __ffs(lanes) - 1;
+        const int bit = __ffs(__shfl_sync(kAll, todo, j)) - 1;
+        const int c = 32 * j + bit;
+        const bool out = warp_suppressed<kHeldR + 1, HIGHER>(J, ww, xc + c, y, __ldg(centre + c));
+        if (lane == j) {
+          todo &= todo - 1u;
+          if (out) m &= ~(1u << bit);
+        }
+      }
+    }
+    if (lane < 4 && width - xc > 32 * lane) {
+      mask[(xc - xs) / 32 + lane] = m;
+      total += __popc(m);
+    }
   }
-  return hit;
+  return __reduce_add_sync(kAll, total);
 }
 
 // The windows of the four pixels x .. x + 3 of a lane at a fixed radius, on
@@ -235,7 +374,7 @@ __device__ __forceinline__ void window_rows(const Job& J, int x, int y, const fl
 // Three rows at a time: 36 registers of loads in flight.
 template <int R, bool HIGHER, int DY = -R>
 __device__ __forceinline__ void window(const Job& J, int x, int y, const float (&s)[4], unsigned& keep) {
-  static_assert(R >= 1 && R <= kLaneR, "one group each side");
+  static_assert(R >= 1 && R <= kGroupR, "one group each side");
   if (keep == 0) return;
   constexpr int kLast = DY + 2 < R ? DY + 2 : R;
   window_rows<R, DY, kLast, HIGHER>(J, x, y, s, keep);
@@ -272,18 +411,24 @@ __device__ __forceinline__ float4 load_chunk(const float* __restrict__ row, int 
   return c;
 }
 
-// One segment: mask words and count.  R = kLaneR + 1 stands for any radius
-// above kLaneR.  The body of a chunk exists once per instance (the candidates
+struct SegmentFlags {
+  uint32_t count;  // pixels that pass
+  unsigned dense;  // bit i: the chunk of columns from 128 i on is left to dense_chunks
+};
+
+// One segment: mask words and count.  R = kHeldR + 1 stands for any radius
+// above kHeldR.  The body of a chunk exists once per instance (the candidates
 // of all four pixel slots share one loop, three chunks are loaded ahead by
 // rotation instead of unrolling): unrolled sixteen-fold the instances
 // outgrew the instruction cache and ran at half this speed.
 template <int R, bool HIGHER, bool VEC>
-__device__ __forceinline__ uint32_t flag_segment(const Job& J, int y, int xs, uint32_t* mask) {
+__device__ __forceinline__ SegmentFlags flag_segment(const Job& J, int y, int xs, uint32_t* mask) {
   constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int end = min(J.width, xs + kSeg);
   const float* row = J.score + static_cast<int64_t>(y) * J.width;
   uint32_t total = 0;
+  unsigned dense = 0;
   WarpWindow ww{};
   if constexpr (R > 0) ww = warp_window(J);
   float4 c = load_chunk<VEC>(row, xs, end), c1 = load_chunk<VEC>(row, xs + kChunk, end);
@@ -295,22 +440,17 @@ __device__ __forceinline__ uint32_t flag_segment(const Job& J, int y, int xs, ui
     unsigned keep = 0;  // bit j: pixel j of this lane passes
 #pragma unroll
     for (int j = 0; j < 4; ++j) keep |= over_threshold<HIGHER>(s[j], J.threshold) ? 1u << j : 0u;
-    if constexpr (R > 0) {
-      unsigned n = __reduce_add_sync(kAll, __popc(keep));
-      if (n > kFew) {
-        constexpr int kR = R <= kLaneR ? R : kFilterR;
-        if constexpr (VEC) {
-          window<kR, HIGHER>(J, xc + 4 * lane, y, s, keep);
-        } else {
-#pragma unroll 1
-          for (int j = 0; j < 4; ++j) {
-            const float sj = j < 2 ? (j == 0 ? s[0] : s[1]) : (j == 2 ? s[2] : s[3]);
-            if (((keep >> j) & 1u) && lane_suppressed<kR, HIGHER>(J, xc + column_of<VEC>(lane, j), y, sj))
-              keep &= ~(1u << j);
-          }
+    unsigned n = 0;
+    if constexpr (R > 0) n = __reduce_add_sync(kAll, __popc(keep));
+    if (n > kFew && !(VEC && R <= kGroupR)) {
+      dense |= 1u << ((xc - xs) / kChunk);
+    } else {
+      if constexpr (VEC && R > 0 && R <= kGroupR) {
+        if (n > kFew) {
+          window<R, HIGHER>(J, xc + 4 * lane, y, s, keep);
+          __syncwarp();
+          n = 0;  // decided
         }
-        __syncwarp();
-        if constexpr (R <= kLaneR) n = 0;  // decided
       }
       if (n > 0) {
         unsigned todo = keep;
@@ -326,41 +466,41 @@ __device__ __forceinline__ uint32_t flag_segment(const Job& J, int y, int xs, ui
           }
         }
       }
-    }
-    uint32_t word[4];  // bit l of word j: column_of(l, j)
+      uint32_t word[4];  // bit l of word j: column_of(l, j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) total += __popc(word[j] = __ballot_sync(kAll, (keep >> j) & 1u));
-    if (lane < 4 && xc + 32 * lane < end) {
-      uint32_t m = 0u;
-      if constexpr (VEC) {  // columns 32 lane + 4i + j come from bit 8 lane + i of word[j]
+      for (int j = 0; j < 4; ++j) total += __popc(word[j] = __ballot_sync(kAll, (keep >> j) & 1u));
+      if (lane < 4 && xc + 32 * lane < end) {
+        uint32_t m = 0u;
+        if constexpr (VEC) {  // columns 32 lane + 4i + j come from bit 8 lane + i of word[j]
 #pragma unroll
-        for (int j = 0; j < 4; ++j) m |= spread4((word[j] >> (8 * lane)) & 0xffu) << j;
-      } else {
-        m = lane < 2 ? (lane == 0 ? word[0] : word[1]) : (lane == 2 ? word[2] : word[3]);
+          for (int j = 0; j < 4; ++j) m |= spread4((word[j] >> (8 * lane)) & 0xffu) << j;
+        } else {
+          m = lane < 2 ? (lane == 0 ? word[0] : word[1]) : (lane == 2 ? word[2] : word[3]);
+        }
+        mask[(xc - xs) / 32 + lane] = m;
       }
-      mask[(xc - xs) / 32 + lane] = m;
     }
     c = c1;
     c1 = c2;
     c2 = c3;
   }
-  return total;
+  return {total, dense};
 }
 
 template <int R, bool HIGHER>
-__device__ __forceinline__ uint32_t flag_radius(const Job& J, int y, int xs, uint32_t* mask) {
+__device__ __forceinline__ SegmentFlags flag_radius(const Job& J, int y, int xs, uint32_t* mask) {
   return J.vec ? flag_segment<R, HIGHER, true>(J, y, xs, mask) : flag_segment<R, HIGHER, false>(J, y, xs, mask);
 }
 
 template <bool HIGHER>
-__device__ __forceinline__ uint32_t flag_dispatch(const Job& J, int y, int xs, uint32_t* mask) {
+__device__ __forceinline__ SegmentFlags flag_dispatch(const Job& J, int y, int xs, uint32_t* mask) {
   switch (J.radius > 0 ? J.radius : 0) {
     case 0: return flag_radius<0, HIGHER>(J, y, xs, mask);
     case 1: return flag_radius<1, HIGHER>(J, y, xs, mask);
     case 2: return flag_radius<2, HIGHER>(J, y, xs, mask);
     case 3: return flag_radius<3, HIGHER>(J, y, xs, mask);
     case 4: return flag_radius<4, HIGHER>(J, y, xs, mask);
-    default: return flag_radius<kLaneR + 1, HIGHER>(J, y, xs, mask);
+    default: return flag_radius<kHeldR + 1, HIGHER>(J, y, xs, mask);
   }
 }
 
@@ -372,7 +512,10 @@ __global__ void __launch_bounds__(kThreads, 4) flags_kernel(const __grid_constan
   const int y = local / J.segs_per_row, xs = (local % J.segs_per_row) * kSeg;
   const int seg = J.seg0 + local;
   uint32_t* mask = b.masks + static_cast<int64_t>(seg) * kWordsPerSeg;
-  const uint32_t n = J.higher ? flag_dispatch<true>(J, y, xs, mask) : flag_dispatch<false>(J, y, xs, mask);
+  const SegmentFlags f = J.higher ? flag_dispatch<true>(J, y, xs, mask) : flag_dispatch<false>(J, y, xs, mask);
+  uint32_t n = f.count;
+  if (f.dense != 0u)
+    n += J.higher ? dense_chunks<true>(J, y, xs, f.dense, mask) : dense_chunks<false>(J, y, xs, f.dense, mask);
   if ((threadIdx.x & 31) == 0) {
     b.counts[seg] = n;
     if (local == 0) b.offsets[seg] = *J.count;  // before emit's last block advances it

@@ -247,3 +247,46 @@ def test_rows_whose_window_spans_more_than_2_31_pixels(hsi, width, radius):
     del score
     torch.cuda.empty_cache()
     assert [(int(d["y"]), int(d["x"])) for d in got] == want and n == len(want)
+
+
+@pytest.mark.parametrize("shape", [(23, 127), (23, 129), (9, 132), (5, 2055), (6, 2180), (1, 300), (300, 3)])
+@pytest.mark.parametrize("radius", [1, 2, 3, 4, 5, 7, 8, 9, 16, 17])
+@pytest.mark.parametrize("higher", [False, True])
+def test_chunk_windows_bit_exact(hsi, orc, shape, radius, higher):
+    """Chunks of 128 columns with more candidates than go one by one, at both sides of the
+    largest radius of a chunk's windows (8) and of the flat single windows (16): columns
+    beside the chunk, at the map's edges and across a row segment (2048), maps lower than the
+    window, ties, NaN and infinities (also the score type's worst, which passes here)."""
+    H, W = shape
+    rng = np.random.default_rng(H * 31 + W + radius)
+    target = rng.integers(0, 8, H * W).astype(np.int32)
+    worst, best = (-np.inf, np.inf) if higher else (np.inf, -np.inf)
+    for levels, share in ((3, 1.0), (60, 1.0), (2000, 0.08)):
+        score = (rng.integers(0, levels, H * W) / levels).astype(np.float32)
+        score[rng.integers(0, H * W, H * W // 30 + 1)] = np.nan
+        score[rng.integers(0, H * W, H * W // 30 + 1)] = worst
+        score[rng.integers(0, H * W, 2)] = best
+        thr = worst if share == 1.0 else (1 - share if higher else share)
+        n0, want = orc.detect(score, target, H, W, thr, radius, higher, capacity=1 << 16)
+        n, got = _gpu_detect(hsi, score, target, H, W, thr, radius, higher, capacity=1 << 16)
+        assert n == n0
+        assert _tuples(got) == _tuples(want)
+
+
+@pytest.mark.parametrize("radius", [2, 3, 6, 12])
+@pytest.mark.parametrize("W", [1024, 1021])
+def test_candidates_per_chunk_bit_exact(hsi, orc, radius, W):
+    """Two to eight candidates a chunk, around the number that still go one by one; some of them
+    neighbours."""
+    H = 70
+    rng = np.random.default_rng(radius + W)
+    score = rng.random((H, W)).astype(np.float32) * 0.5
+    for y in range(H):
+        for x0 in range(0, W, 128):
+            n = 2 + (y + x0 // 128) % 7
+            at = x0 + rng.integers(0, min(128, W - x0), n)
+            score[y, at] = 0.9 + 0.01 * rng.integers(0, 8, n)
+    n0, want = orc.detect(score.reshape(-1), None, H, W, 0.9, radius, True, capacity=1 << 16)
+    n, got = _gpu_detect(hsi, score, None, H, W, 0.9, radius, True, capacity=1 << 16)
+    assert n == n0
+    assert _tuples(got) == _tuples(want)

@@ -1268,12 +1268,19 @@ int launch_form(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaStream
 template <typename T, int KS, int KC>
 int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaStream_t stream) {
   // Sixteen filters of a pixel keep the FP32 scorer on the banks' shared-memory
-  // reads, which the wide form halves: it takes 0.85 to 0.93 of the narrow
-  // form's time a pixel (four 1024 x 1024 x 113 frames 427 us, 459; 2 x 1024 x
-  // 1024 x 224 384, 441).  Its tiles are larger, so a short launch can leave more
-  // of the SMs' last round empty (640 x 640 x 113: 63 us, 60): it is taken when the
-  // busiest SM's pixels are at most 1.15 times the narrow form's.  Frames in a
-  // device table have unknown sizes here and take the narrow form.
+  // reads, which the wide form halves: it takes 0.86 to 0.95 of the narrow
+  // form's time on long launches (eight 1024 x 1024 x 113 frames 841 us, 913;
+  // 2116 x 2116 x 224 801, 933).  It has two CTAs of seven warps on an SM where
+  // the narrow form has three of eight, and larger tiles, so short launches
+  // depend on how the tiles fall on the SMs:
+  // - at most a tile per SM leaves each alone with too few warps: 362 x 362 x 224
+  //   56 us, 41; 148 tiles of 113 bands 31, 29 (two per SM 36, 45);
+  // - an odd number of tiles on nearly every SM ends with such a lone one (three
+  //   62 us, 59; five 89, 84; a third tile on two SMs of three 48, 58), which is
+  //   lost among nine and more;
+  // - the busiest SM's pixels may be up to 1.15 times the narrow form's (640 x
+  //   640 x 113: 63 us, 60).
+  // Frames in a device table have unknown sizes here and take the narrow form.
   if constexpr (sizeof(T) == 4 && fused_banks<KS, KC>() && KS + KC == 16) {
     int64_t wide = 0, narrow = 0;  // tiles
     if (!p.table)
@@ -1282,9 +1289,9 @@ int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaSt
         wide += div_up<int64_t>(P, tile_px<true>());
         narrow += div_up<int64_t>(P, tile_px<false>());
       }
-    const int64_t sms = sm_count();
-    if (wide > 0 &&
-        100 * div_up(wide, sms) * tile_px<true>() <= 115 * div_up(narrow, sms) * tile_px<false>())
+    const int64_t sms = sm_count(), turns = div_up(wide, sms);
+    const bool lone = turns % 2 == 1 && turns < 9 && 100 * (wide - (turns - 1) * sms) > 95 * sms;
+    if (wide > sms && !lone && 100 * turns * tile_px<true>() <= 115 * div_up(narrow, sms) * tile_px<false>())
       return launch_form<T, KS, KC, true>(p, max_bands, ctas_per_sm, stream);
   }
   return launch_form<T, KS, KC, false>(p, max_bands, ctas_per_sm, stream);

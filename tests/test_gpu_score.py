@@ -10,6 +10,8 @@ bits.  Tolerances (stated here, checked below):
                (bench/bench_sam.cu:156-183);
   CEM        : |gpu - oracle| <= 1e-5 * sum_b |w_b x_b| + 1e-6.
 """
+import re
+
 import numpy as np
 import pytest
 import torch
@@ -362,6 +364,71 @@ def test_wide_form_equals_narrow_form(hsi, shapes, B, ks, kc):
     for a, b in zip(out[::2], out[1::2]):
         for key in a[2]:
             assert torch.equal(a[2][key], b[2][key]), key
+
+
+def _scorer_forms(fn):
+    """Whether each scorer kernel that a captured call launches is the wide form
+    (score_kernel's last template argument)."""
+    from cuda.bindings import driver, runtime
+    stream = torch.cuda.Stream()
+    stream.wait_stream(torch.cuda.current_stream())
+    fn(stream)  # one-time set-up
+    stream.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph, stream=stream):
+        fn(stream)
+    g = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    _, _, n = runtime.cudaGraphGetNodes(g)
+    err, nodes, n = runtime.cudaGraphGetNodes(g, n)
+    assert err == runtime.cudaError_t.cudaSuccess
+    forms = []
+    for node in nodes[:n]:
+        if runtime.cudaGraphNodeGetType(node)[1] != runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel:
+            continue
+        err, params = driver.cuGraphKernelNodeGetParams(driver.CUgraphNode(int(node)))
+        assert err == driver.CUresult.CUDA_SUCCESS
+        if int(params.func):
+            err, name = driver.cuFuncGetName(params.func)
+        else:
+            err, name = driver.cuKernelGetName(params.kern)
+        assert err == driver.CUresult.CUDA_SUCCESS
+        m = re.search(r"score_kernelI.*Lb([01])EE", name.decode())
+        if m:
+            forms.append(m.group(1) == "1")
+    return forms
+
+
+def _sixteen_filters(hsi, pixels, B, gen):
+    """Frames of one row each, eight SAM targets and eight CEM filters."""
+    frames, keep = [], []
+    for P in pixels:
+        cube = torch.rand((B, (P + 31) // 32 * 32), generator=gen, device="cuda")
+        sam = torch.rand((8, B), generator=gen, device="cuda")
+        cem = torch.randn((8, B), generator=gen, device="cuda")
+        norms = sam.double().square().sum(1).sqrt().float()
+        best, which = torch.empty((2, P), device="cuda"), torch.empty((2, P), dtype=torch.int32, device="cuda")
+        frames.append(hsi.make_frame(cube, 1, P, B, sam_targets=sam, sam_norms=norms, cem_weights=cem,
+                                     sam_best=best[0], sam_best_target=which[0], cem_best=best[1],
+                                     cem_best_target=which[1], map_stride=P))
+        keep.append((cube, sam, cem, norms, best, which))
+    return frames, keep
+
+
+@pytest.mark.parametrize("tiles, wide", [(0.3, False), (0.99, False), (1.8, True), (1.99, True), (2.02, False),
+                                         (2.7, True), (2.99, False), (3.9, True), (4.99, False), (7.9, True),
+                                         (9.0, True), (20.5, True)])
+def test_wide_form_where_its_tiles_fill_the_gpu(hsi, tiles, wide):
+    """The scorer's form at so many 896-pixel tiles per SM, in one frame and in four."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    gen = torch.Generator(device="cuda").manual_seed(1)
+    n = int(tiles * sms)
+    for pixels in ([n * 896 - 3], [n // 4 * 896, n // 4 * 896, n // 4 * 896, (n - 3 * (n // 4)) * 896]):
+        frames, keep = _sixteen_filters(hsi, pixels, 4, gen)
+        assert _scorer_forms(lambda s: hsi.score_frames(frames, stream=s)) == [wide], pixels
+    table = hsi.frame_table(frames)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    assert _scorer_forms(lambda s: hsi.score_frames_device(table, 4, max_bands=4, max_sam=8, max_cem=8, status=status,
+                                                           stream=s)) == [False]
 
 
 def test_device_table_rejects_frames_outside_bounds(hsi):

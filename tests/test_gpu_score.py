@@ -431,6 +431,49 @@ def test_wide_form_where_its_tiles_fill_the_gpu(hsi, tiles, wide):
                                                            stream=s)) == [False]
 
 
+@pytest.mark.parametrize("specs", [
+    # (height, width, bands, SAM targets, CEM filters) of each frame
+    [(300, 301, 31, 8, 8), (7, 5, 113, 1, 8), (299, 399, 31, 8, 3), (1, 896, 8, 0, 5), (1, 897, 9, 8, 0), (60, 300, 113, 7, 7)],
+    [(1, 260 * 896 + 1, 224, 8, 8)],
+    [(257, 700, 224, 8, 8), (120, 400, 7, 8, 8)],
+    [(300, 400, 17, 16, 0), (300, 400, 33, 12, 0), (31, 33, 64, 1, 0)],
+    [(300, 400, 17, 0, 16), (300, 400, 33, 0, 9), (31, 33, 64, 0, 1)],
+])
+def test_wide_form_equals_narrow_form_over_frames(hsi, specs):
+    """As above where the launch does take the wide form (checked), over frames of different
+    sizes, bands and banks: the bank and the tile ring are carried from frame to frame."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    assert sms == 148, "the sizes put 1.1 to 2 tiles on each of 148 SMs"
+    gen = torch.Generator(device="cuda").manual_seed(sum(b for _, _, b, _, _ in specs))
+    frames, out, keep = ([], []), ([], []), []
+    for n, (H, W, B, ks, kc) in enumerate(specs):
+        P = H * W
+        cube = torch.rand((B, (P + 7) // 8 * 8), generator=gen, device="cuda")
+        sam = torch.rand((max(ks, 1), B), generator=gen, device="cuda")
+        cem = torch.randn((max(kc, 1), B), generator=gen, device="cuda")
+        norms = sam.double().square().sum(1).sqrt().float()
+        keep.append((cube, sam, cem, norms))
+        for form in (0, 1):
+            maps = torch.full((ks + kc, P + n), -7.0, device="cuda")
+            best = torch.full((2, P), -7.0, device="cuda")
+            which = torch.full((2, P), -7, dtype=torch.int32, device="cuda")
+            frames[form].append(hsi.make_frame(
+                cube, H, W, B, map_stride=P + n,
+                **(dict(sam_targets=sam, sam_norms=norms, sam_maps=maps, sam_best=best[0], sam_best_target=which[0])
+                   if ks else {}),
+                **(dict(cem_weights=cem, cem_maps=maps[ks:], cem_best=best[1], cem_best_target=which[1]) if kc else {})))
+            out[form].extend([maps, best, which])
+    assert _scorer_forms(lambda s: hsi.score_frames_batch(frames[0], stream=s)) == [True]
+    hsi.score_frames_batch(frames[0])
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    hsi.score_frames_device(hsi.frame_table(frames[1]), len(specs), max_bands=max(s[2] for s in specs),
+                            max_sam=max(s[3] for s in specs), max_cem=max(s[4] for s in specs), status=status)
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    for a, b in zip(*out):
+        assert torch.equal(a, b)
+
+
 def test_device_table_rejects_frames_outside_bounds(hsi):
     """A frame with more bands than the launch allows is skipped, not overrun."""
     H, W, B = 8, 8, 64

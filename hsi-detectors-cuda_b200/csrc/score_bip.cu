@@ -30,6 +30,8 @@
 // cube.  All targets are scored from shared memory in one pass over HBM
 // (groups of 8 or 16, two targets per packed FMA, the bank zero-padded to the
 // group).
+#include <algorithm>
+
 #include "common.cuh"
 #include "launch_state.h"
 #include "sam_math.cuh"
@@ -144,9 +146,15 @@ __device__ __forceinline__ void band_loop(const float* xr, const float* tgc, int
   }
 }
 
+// Blocks of max_warps whose registers fit an SM.
+template <int G, bool kTwo>
+constexpr int full_blocks() {
+  return !kTwo ? 1 : G == 8 ? 4 : 3;
+}
+
 // kTwo: two tile buffers a warp.
 template <int G, int V, bool kTwo>
-__global__ void __launch_bounds__(max_warps(kTwo) * 32, !kTwo ? 1 : G == 8 ? 4 : 3) sam_bip_kernel(const BipArgs a) {
+__global__ void __launch_bounds__(max_warps(kTwo) * 32, full_blocks<G, kTwo>()) sam_bip_kernel(const BipArgs a) {
   extern __shared__ __align__(16) float sm[];
   const int B = a.bands, T = a.targets, TP = (T + G - 1) / G * G, S = row_stride(B);
   float* tg = sm;                  // [b][TP], zero beyond T
@@ -235,19 +243,29 @@ template <int G, int V, bool kTwo>
 int launch_bip_k(const BipArgs& a, cudaStream_t stream) {
   const size_t fixed = bip_fixed_bytes(a.bands, a.targets), per_warp = bip_warp_bytes(a.bands) * (kTwo ? 2 : 1);
   const int64_t ntiles = div_up<int64_t>(a.pixels, kPx);
-  // the block size that keeps most warps on an SM (1 KB of each block's shared memory is the system's)
+  // the block size that keeps most warps on an SM, as shared memory (1 KB of each
+  // block's is the system's) and registers allow (seven warps a block by shared
+  // memory alone: 520 x 696 x 16 with 16 targets 14.4 us, 12.8 on eight).  With two
+  // buffers a smaller block has to keep a quarter more (31 bands, one target:
+  // seven warps 12.5 us, eight 11.9).
+  constexpr size_t kRegisterWarps = static_cast<size_t>(full_blocks<G, kTwo>()) * max_warps(kTwo);
   int warps = 1;
   size_t most = 0;
   for (int w = max_warps(kTwo); w >= 1; --w) {
     const size_t block = fixed + w * per_warp;
-    const size_t on_sm = block > kSmemCap ? 0 : w * ((kSmemCap + 1024) / (block + 1024));
-    if (on_sm > most) {
-      most = on_sm;
+    const size_t blocks =
+        block > kSmemCap ? 0 : std::min((kSmemCap + 1024) / (block + 1024), kRegisterWarps / static_cast<size_t>(w));
+    if (w * blocks > most + (kTwo ? most / 4 : 0)) {
+      most = w * blocks;
       warps = w;
     }
   }
-  // few tiles: over all SMs, but four warps a block share the staging of the bank
+  // few tiles: over all SMs, but four warps a block share the staging of the bank;
+  // where one block fills an SM, no more warps than its rounds of tiles need (250 x
+  // 331 x 98 with 8 targets, 18 tiles per SM: 11.4 us on nine warps, 16.1 on sixteen)
   const int64_t over_sms = div_up<int64_t>(ntiles, device_sm_count());
+  if (most == static_cast<size_t>(warps) && over_sms > warps)
+    warps = static_cast<int>(div_up<int64_t>(over_sms, div_up<int64_t>(over_sms, warps)));
   const int64_t spread = over_sms > 4 ? over_sms : 4;
   if (warps > spread) warps = static_cast<int>(spread);
   const size_t smem = fixed + static_cast<size_t>(warps) * per_warp;

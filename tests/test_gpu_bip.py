@@ -81,6 +81,14 @@ def test_bip_many_tiles_per_warp(hsi, orc, H, W, B, T, off):
     test_bip_equals_bsq_bit_for_bit(hsi, orc, H, W, B, T, off)
 
 
+@pytest.mark.parametrize("H,W,B,T", [(250, 331, 98, 8), (273, 278, 113, 9), (273, 295, 224, 16), (137, 137, 64, 16),
+                                     (94, 102, 96, 1)])
+def test_bip_blocks_that_follow_the_tiles(hsi, orc, H, W, B, T):
+    """A few more tiles per SM than a block has warps, so that the block takes fewer warps
+    and several rounds (18, 17, 18, 5 and 3 tiles per SM)."""
+    test_bip_equals_bsq_bit_for_bit(hsi, orc, H, W, B, T, 0)
+
+
 def test_bip_pixel_equal_to_a_target_scores_zero(hsi):
     H, W, B, T = 8, 8, 20, 3
     rng = np.random.default_rng(5)

@@ -245,7 +245,9 @@ struct PieceWalk {
   __device__ int64_t hi(int f) const { return min(kb1, t.f[f].kb_begin + frame_kb(t.f[f])); }
 };
 
-template <typename T>
+// kAhead: a converter warp loads its four rows before it converts any; without, row
+// by row.  The group's largest band count picks one (launch_tensor_group).
+template <typename T, bool kAhead>
 __global__ void __launch_bounds__(kThreads, 1) stats_gemm_kernel(const __grid_constant__ GemmParams p) {
   const FrameTable& t = p.t;
   const int64_t kb0 = t.total_kb * blockIdx.x / gridDim.x;
@@ -486,11 +488,13 @@ __global__ void __launch_bounds__(kThreads, 1) stats_gemm_kernel(const __grid_co
       auto convert_half = [&](auto full, const T* in, int sub_off, unsigned char* op, int half, int nvalid) {
         Raw4<T> raw[kSlots];
 #pragma unroll
-        for (int t2 = 0; t2 < kSlots; ++t2) raw[t2] = load_raw4<T>(in + (band0 + 32 * t2) * kBoxPx + sub_off + lp);
+        for (int t2 = 0; kAhead && t2 < kSlots; ++t2)
+          raw[t2] = load_raw4<T>(in + (band0 + 32 * t2) * kBoxPx + sub_off + lp);
 #pragma unroll
         for (int t2 = 0; t2 < kSlots; ++t2) {
           const uint32_t o = (o0 + 4096u * t2) ^ (half ? 64u : 0u);
           if (is_band[t2]) {
+            if (!kAhead) raw[t2] = load_raw4<T>(in + (band0 + 32 * t2) * kBoxPx + sub_off + lp);
             const float4 x = to_f4(raw[t2]);
             const float xv[4] = {x.x, x.y, x.z, x.w};
             uint32_t y[4];
@@ -1534,16 +1538,23 @@ int launch_tensor_group(const hsi_moments_job* const* jobs, int m, void* workspa
   }
   if (used > kMaxCtas + m) return HSI_E_CAPACITY;  // cannot happen: pieces <= CTAs + frames - 1
   const StatsSmem L = stats_smem<T>();
-  // set once per device and element type
-  const cudaError_t configured = raise_smem_limit(stats_gemm_kernel<T>, static_cast<int>(L.total));
+  // FP32 frames of up to 31 bands (with the ones row, the first of a converter warp's
+  // four rows alone): most rows that a warp would load ahead lie past the bands.  8 x
+  // 1024 x 1024 x 4: 500 us row by row, 515 ahead; 24 bands 500 and 523.  FP16 rows are
+  // half as long, and loading them ahead costs nothing (486 and 484).
+  auto gemm = stats_gemm_kernel<T, true>;
+  if constexpr (sizeof(T) == 4)
+    if (t.max_bands < 32) gemm = stats_gemm_kernel<T, false>;
+  // set once per device and instance
+  const cudaError_t configured = raise_smem_limit(gemm, static_cast<int>(L.total));
   if (configured != cudaSuccess) return static_cast<int>(configured);
   launch_shift<T>(t, s);
   p.conditional = 0;
-  stats_gemm_kernel<T><<<grid, kThreads, L.total, s>>>(p);
+  gemm<<<grid, kThreads, L.total, s>>>(p);
   range_kernel<T><<<4 * num_sms(), 256, 0, s>>>(t);
   rescale_kernel<<<m, 128, 0, s>>>(t);
   p.conditional = 1;
-  stats_gemm_kernel<T><<<grid, kThreads, L.total, s>>>(p);
+  gemm<<<grid, kThreads, L.total, s>>>(p);
   int most = 0;
   for (int f = 0; f < m; ++f) most = t.f[f].nslots > most ? t.f[f].nslots : most;
   if (most > 32)

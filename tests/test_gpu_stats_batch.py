@@ -181,3 +181,15 @@ def test_split_path_with_caller_reference(hsi, orc):
     got = _run_batch(hsi, [(B, H, W, 0)], [cube], refs=[ref])[0]
     cov, mean = _cov_err(hsi, orc, cube, got, B, H * W)
     assert cov < 5e-8 and mean < 1e-7, (cov, mean)
+
+
+@pytest.mark.parametrize("bands", [1, 23, 31, 32])
+@pytest.mark.parametrize("shape", [(181, 190), (256, 128)])
+def test_few_bands_alone_equal_few_bands_beside_many(hsi, bands, shape):
+    """FP32 frames of up to 31 bands are converted row by row, in a group with larger band
+    counts four rows at a time: the same bits."""
+    specs = [(bands, *shape, 0), (113, 200, 200, 0)]
+    cubes = [_frame(hsi, B, H, W, dt, 0x5EED7300 + B) for B, H, W, dt in specs]
+    alone = _run_batch(hsi, specs[:1], cubes[:1])
+    beside = _run_batch(hsi, specs, cubes)
+    assert torch.equal(alone[0], beside[0])

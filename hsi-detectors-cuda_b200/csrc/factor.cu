@@ -892,6 +892,15 @@ __host__ __device__ inline size_t own_doubles(int B) {
   return vectors + (B <= kTileMaxBands ? tri(B) : B <= kSmemMaxBands ? 2 * tri(B) : 0);
 }
 
+// The three factorisations, by the band count.  Each has a kernel of its own: run
+// once, a small factorisation is bound by instruction fetches, which code of the
+// others in between makes more of (16 bands, no targets: 8.4 us in one kernel, 7.9;
+// a single band with 16 targets 5.5 and 5.0).
+enum class Path { kTiles, kInplace, kBlocked };
+Path path_of(int B) {
+  return B <= kTileMaxBands ? Path::kTiles : B > kSmemMaxBands && B <= kHybridMaxBands ? Path::kInplace : Path::kBlocked;
+}
+
 // One cluster of two CTAs per frame, on two SMs at once:
 //   rank 0: covariance S = L L^T -> mean, whitener W = L^-1, ACE vectors;
 //   rank 1: correlation R = C C^T -> CEM weights (only when there are targets).
@@ -899,6 +908,7 @@ __host__ __device__ inline size_t own_doubles(int B) {
 // rank 1 writes its result code into rank 0's shared memory and rank 0 writes
 // the frame's status: an empty frame or a covariance that is not positive
 // definite first (the reference stops there), else the correlation's code.
+template <Path kPath>
 __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_kernel(const FactorArgs args) {
   namespace cg = cooperative_groups;
   extern __shared__ __align__(16) double smem[];
@@ -913,8 +923,8 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   double* out64 = args.stats64 ? args.stats64 + f * per : nullptr;
   float* out32 = args.stats32 ? args.stats32 + f * per : nullptr;
   float* cem32 = args.cem32 ? args.cem32 + static_cast<size_t>(f) * T * B : nullptr;
+  constexpr bool tiles = kPath == Path::kTiles, inplace = kPath == Path::kInplace;
   const bool in_smem = B <= kSmemMaxBands;
-  const bool inplace = !in_smem && B <= kHybridMaxBands;
   // smem: mean[B], two products of W with a target chunk (kChunk x B each), the
   // panel / block-row buffer, the diagonal block's inverse, then the packed
   // matrices (in the workspace when B is large) and the targets' stage.  The
@@ -927,11 +937,10 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   double* vs = lp + lp_elems(B);
   double* cbuf = vs + kNb * kNb;  // the tile path's panel, Dinv and flag (kTileShared doubles, 16-byte aligned)
   // the tile path keeps the factor in registers: only W lives in shared memory
-  const bool tiles = B <= kTileMaxBands;
   double* ws = args.scratch + (static_cast<size_t>(f) * 2 + chain) * 2 * tri(B);
   double* A = in_smem ? cbuf + kTileShared : ws;
   double* W = tiles ? A : A + tri(B);
-  if (inplace) {
+  if constexpr (inplace) {
     vs = mean + B;
     A = W = vs + kNb * kNb;
     xs = ws;
@@ -942,7 +951,7 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
   // buffer, or the diagonal block's inverse when that buffer is in the workspace
   int span = kStageBands;
   size_t stage_at = own_doubles(B);
-  if (inplace) {
+  if constexpr (inplace) {
     const bool room = inplace_tb_in_smem(B);
     stage_at = room ? B + kNb * kNb + tri(B) : B;
     if (!room) span = 12;  // 192 of kNb * kNb doubles
@@ -963,9 +972,9 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
     __syncthreads();
     // covariance (chain 0) or correlation (chain 1), loaded (src/linalg.cpp:56-79)
     bool factored;
-    if (tiles) {
+    if constexpr (tiles) {
       factored = chol_inv_tiles(outer, mean, N, args.loading, chain == 0, W, B, cbuf);
-    } else if (inplace) {
+    } else if constexpr (inplace) {
       // pointers taken straight from the shared array, so the inlined loops
       // address shared memory directly
       double* As = smem + B + kNb * kNb;
@@ -1073,7 +1082,7 @@ __global__ void __cluster_dims__(1, 2, 1) __launch_bounds__(kThreads) factor_ker
 }
 
 size_t smem_bytes(int B) {
-  if (B > kSmemMaxBands && B <= kHybridMaxBands)
+  if (path_of(B) == Path::kInplace)
     return sizeof(double) * (inplace_core(B) + (inplace_tb_in_smem(B) ? kNb * last_block_row(B) : 0));
   return sizeof(double) * (own_doubles(B) + 1 + kStageBands * kChunk);
 }
@@ -1122,8 +1131,12 @@ extern "C" HSI_API int hsi_build_statistics(int num_frames, int bands, int num_t
   a.scratch = static_cast<double*>(d_workspace);
   const size_t smem = smem_bytes(bands);
   if (smem > 227 * 1024) return HSI_E_CAPACITY;
-  const cudaError_t e = raise_smem_limit(factor_kernel, static_cast<int>(smem));
+  const Path path = path_of(bands);
+  const auto kernel = path == Path::kTiles     ? factor_kernel<Path::kTiles>
+                      : path == Path::kInplace ? factor_kernel<Path::kInplace>
+                                               : factor_kernel<Path::kBlocked>;
+  const cudaError_t e = raise_smem_limit(kernel, static_cast<int>(smem));
   if (e != cudaSuccess) return static_cast<int>(e);
-  factor_kernel<<<dim3(num_frames, 2), kThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(a);
+  kernel<<<dim3(num_frames, 2), kThreads, smem, reinterpret_cast<cudaStream_t>(stream)>>>(a);
   return static_cast<int>(cudaGetLastError());
 }

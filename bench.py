@@ -835,9 +835,9 @@ def extra_records(args, device, line):
 
 # DRAM bytes (read + write) per frame of the scoring kernel, from the ncu
 # captures summarised in profiles/ (score_kernel_samcem8_f32_4x1024x1024x113.md:
-# 2.250 GB for a 4-frame launch; rxace_tc_kernel_f32_2048x1024x113.md: one
+# 2.216 GB for a 4-frame launch; rxace_tc_kernel_f32_2048x1024x113.md: one
 # frame).  The scorer's traffic grows with the frames in the launch.
-TRAFFIC_PER_FRAME = {"sam_cem": 562.52e6, "rx_ace": 1036.90e6}
+TRAFFIC_PER_FRAME = {"sam_cem": 554.08e6, "rx_ace": 1035.63e6}
 
 
 def load_traffic(workload, frames):

@@ -782,11 +782,11 @@ namespace {
 constexpr int kNoAllocSegs = HSI_DETECT_NOALLOC_MAX_SEGMENTS;
 constexpr size_t kNoAllocBytes = static_cast<size_t>(kNoAllocSegs) * sizeof(uint32_t) * (2 + kWordsPerSeg) + 256;
 
-// Segment counts, offsets and ballot masks of one call.  Every word a call
-// reads is written earlier by that same call (flags writes every mask word
-// that covers pixels of the map, and scan and emit read no other; scan writes
-// the counts and offsets), so nothing here needs to start at zero and stale
-// contents from a previous call are never read.
+// Segment counts, the map's offset and ballot masks of one call.  Every word a
+// call reads is written earlier by that same call (flags writes the counts, the
+// map's offset and every mask word that covers pixels of the map, and emit reads
+// no other; maps of this size have no scan launch), so nothing here needs to
+// start at zero and stale contents from a previous call are never read.
 static __device__ __align__(256) uint32_t g_noalloc_scratch[kNoAllocBytes / sizeof(uint32_t)];
 
 constexpr int kNoAllocMaxDevices = 64;

@@ -24,10 +24,10 @@
 // target vectors in the caller's workspace), and beyond that the matrices
 // live in the workspace.  The solves use the explicit inverses.
 // What bounds it is latency: one warp's diagonal blocks, the block barriers and
-// the solves.  224 bands and 16 targets, both chains: 310 us (430 with the
+// the solves.  224 bands and 16 targets, both chains: 288 us (402 with the
 // diagonal's update and inverse as chains of one warp, a lane per row and
 // target in the solves, and 64-bit divisions for every output index); 113
-// bands and 8 targets 60 us.
+// bands and 8 targets 56 us (60).
 // Tried: two diagonal blocks through the register tiles and every product on
 // the FP64 tensor pipe (mma.sync m8n8k4) took 218 us at 224 bands.  Its sums
 // run in another order, so the FP32 weights that the scorers make of them round

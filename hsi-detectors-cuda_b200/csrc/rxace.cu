@@ -29,8 +29,8 @@
 // leaves the other's latencies bare).  The squares of groups G, G + 16, G + 32
 // form one partial sum of RX; a pair waits for the pair eight before it, which
 // is always started earlier, before it adds its own.
-// Bound: FP32 FMA (B^2 / 2 + T B per pixel; the pipe is 71 % busy) and the
-// shared-memory reads beside it (74 %: eight weights and four pixels per lane
+// Bound: FP32 FMA (B^2 / 2 + T B per pixel; the pipe is 72 % busy) and the
+// shared-memory reads beside it (71 %: eight weights and four pixels per lane
 // for 16 packed FMAs; sixteen rows by two pixels needed ten wavefronts where
 // this tile needs eight, and was 13 % slower).  1024 x 1024 x 224 fp16, 16
 // targets: 1.28 ms; 3.24 with 128 x 128 tiles that staged W and the cube per

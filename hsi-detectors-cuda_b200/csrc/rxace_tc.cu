@@ -34,8 +34,9 @@
 //               output rows 0-63, four for rows 64-127
 // Two MMA rounds per tile, each into its own half of TMEM: round h covers rows
 // [32h, 32h + 32) and [64 + 32h, 64 + 32h + 32), so that both sets of epilogue
-// warps drain it at once; they give its columns back as soon as the values are
-// in registers, and the next round's products run under their arithmetic.
+// warps drain it at once.  They give its columns back after the arithmetic of its
+// last eight columns; the other round's products run under that arithmetic, and the
+// next tile's under the output of the targets.
 // Round h writes S0 to columns [256h, 256h + 64), S1 the next 64, S2 and S3
 // after them.  The whitener limbs lie in shared memory by round, [M0 | M1 | M2]
 // of its 64 rows (8 KB each).  Bands are padded to a multiple of 32 only: short
@@ -45,7 +46,7 @@
 // the converters and the epilogue's row constants, about 4900 of the 5500 cycles
 // that a 128-pixel tile takes at 113 bands.  2048 x 1024 x 113 FP32 with 8 targets:
 // 340 us; 391 us when each half of TMEM was drained by four warps alone and held
-// to the end, an operand was read by five instructions per 32 bands, and the
+// until the tile's output, an operand was read by five instructions per 32 bands, and the
 // epilogue's output took the targets one at a time.  1024 x 1024 x 16: 95 us,
 // 154 us before.
 #include <cuda_fp16.h>

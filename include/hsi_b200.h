@@ -316,8 +316,8 @@ HSI_API int hsi_detect(const float* d_score, const int32_t* d_target, int height
                        size_t workspace_bytes, hsi_stream_t stream);
 
 /* The same for up to 64 score maps in two launches for the whole batch (three
- * when a map has more than 16384 rows or segments of 2048 pixels).  Job descriptors live in host memory; the pointers in them
- * are device pointers. */
+ * when a map has more than 16384 row segments of 2048 pixels).  Job descriptors
+ * live in host memory; the pointers in them are device pointers. */
 typedef struct hsi_detect_job {
   const float* score;
   const int32_t* target;     /* nullable */
@@ -460,8 +460,9 @@ HSI_API int hsi_accumulate_shifted_moments(const double* d_moments, const float*
  *    append offset the caller sets (normally zero) before the call;
  *  - the first call on each device does a one-time set-up (it looks up the
  *    array's device address in the current context), so that first call should
- *    come before any stream capture; the set-up runs again after the device's context is re-created
- *    (for example by cudaDeviceReset), since the array may then move.
+ *    come before any stream capture; the set-up runs again after the device's
+ *    context is re-created (for example by cudaDeviceReset), since the array may
+ *    then move.
  * It calls no allocating routine.  HSI_E_NO_DEVICE for device ordinals >= 64. */
 #define HSI_DETECT_NOALLOC_MAX_SEGMENTS 8192
 HSI_API int hsi_detect_noalloc(const float* d_score, const int32_t* d_target, int height, int width,

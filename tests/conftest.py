@@ -18,6 +18,19 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (B200, sm_100a)")
 
 
+# Tests that fail where the reference's own library (oracle/_ref, compiled from its sources)
+# is not built.
+NEEDS_REFERENCE = ("test_cpp_threshold.py", "test_gpu_cli_parity.py", "test_gpu_parity_configs.py",
+                   "test_lagged_stream_matches_oracle_with_previous_statistics")
+
+
+def pytest_collection_modifyitems(config, items):
+    """Where that library is missing they run last, so that `-x` stops behind all others."""
+    import oracle
+    if not oracle.ref_available():
+        items.sort(key=lambda item: any(name in item.nodeid for name in NEEDS_REFERENCE))
+
+
 @pytest.fixture(scope="session")
 def golden():
     return np.load(GOLDEN, allow_pickle=False)

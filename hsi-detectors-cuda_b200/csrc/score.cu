@@ -1275,9 +1275,10 @@ int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaSt
   // depend on how the tiles fall on the SMs:
   // - at most a tile per SM leaves each alone with too few warps: 362 x 362 x 224
   //   56 us, 41; 148 tiles of 113 bands 31, 29 (two per SM 36, 45);
-  // - an odd number of tiles on nearly every SM ends with such a lone one (three
-  //   62 us, 59; five 89, 84; a third tile on two SMs of three 48, 58), which is
-  //   lost among nine and more;
+  // - an odd number of tiles on most SMs ends with such lone ones (three 62 us, 59;
+  //   five 89, 84; 4.83 per SM 86, 83).  That begins where some SM gets two of them in
+  //   a row, between 104 and 111 of 148 (4.73 per SM 74, 84; 2.70 48, 58; 2.75 62,
+  //   58), and is lost among nine tiles and more;
   // - the busiest SM's pixels may be up to 1.15 times the narrow form's (640 x
   //   640 x 113: 63 us, 60).
   // Frames in a device table have unknown sizes here and take the narrow form.
@@ -1290,7 +1291,7 @@ int launch_instance(const ScoreParams& p, int max_bands, int ctas_per_sm, cudaSt
         narrow += div_up<int64_t>(P, tile_px<false>());
       }
     const int64_t sms = sm_count(), turns = div_up(wide, sms);
-    const bool lone = turns % 2 == 1 && turns < 9 && 100 * (wide - (turns - 1) * sms) > 95 * sms;
+    const bool lone = turns % 2 == 1 && turns < 9 && 100 * (wide - (turns - 1) * sms) > 72 * sms;
     if (wide > sms && !lone && 100 * turns * tile_px<true>() <= 115 * div_up(narrow, sms) * tile_px<false>())
       return launch_form<T, KS, KC, true>(p, max_bands, ctas_per_sm, stream);
   }

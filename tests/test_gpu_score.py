@@ -415,7 +415,7 @@ def _sixteen_filters(hsi, pixels, B, gen):
 
 
 @pytest.mark.parametrize("tiles, wide", [(0.3, False), (0.99, False), (1.8, True), (1.99, True), (2.02, False),
-                                         (2.7, True), (2.99, False), (3.9, True), (4.99, False), (7.9, True),
+                                         (2.7, True), (2.8, False), (2.99, False), (3.9, True), (4.83, False), (7.9, True),
                                          (9.0, True), (20.5, True)])
 def test_wide_form_where_its_tiles_fill_the_gpu(hsi, tiles, wide):
     """The scorer's form at so many 896-pixel tiles per SM, in one frame and in four."""
